@@ -134,9 +134,8 @@ struct DftArgs {
     long long frame_stride, row_pitch;
     int bpp, pixmode, x_off, y_off;
     float2 *ring;
-    long long E;
+    RingLayout lay;
     long long first_label;
-    int R;
     int nframes;
     FftScale sc;
     const uint4 *tables;  // dft_table_bytes(s) bytes, already in the shared-memory layout
@@ -348,13 +347,14 @@ __global__ void __launch_bounds__(kDftThreads, 1) dft_bf16_kernel(DftArgs a) {
                 }
             }
             __syncthreads();
-            const long long slot = (a.first_label + f) % a.R;
+            const FramePtr frame(a.ring, a.lay, static_cast<int>((a.first_label + f) % a.lay.R));
             const int ntl = tiles - b * TPB < TPB ? tiles - b * TPB : TPB;
-            // sc.n = S * NX is even and every tile starts on a 16-byte boundary of the ring slot
-            uint4 *dst = reinterpret_cast<uint4 *>(a.ring + slot * a.E + sc.off + static_cast<long long>(b * TPB) * sc.n);
+            // sc.n = S * NX is even: every tile starts at an even element, and pairs of elements are
+            // 16 aligned bytes of one element block
+            const int dst = static_cast<int>(sc.off + static_cast<long long>(b * TPB) * sc.n);
             const uint4 *src = reinterpret_cast<const uint4 *>(stage);
             const int n16 = ntl * S * NX / 2;
-            for (int i = tid; i < n16; i += kDftThreads) dst[i] = src[i];
+            for (int i = tid; i < n16; i += kDftThreads) *reinterpret_cast<uint4 *>(frame.at(dst + 2 * i)) = src[i];
         }
         tc_fence_before();
         __syncthreads();

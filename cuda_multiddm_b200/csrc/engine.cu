@@ -31,6 +31,7 @@
 #include "kernels.cuh"
 #include "lag.cuh"
 #include "engine_internal.hpp"
+#include "lag_hist_host.hpp"
 #include "lag_host.hpp"
 #include "pinned_pool.hpp"
 #include "stream_pool.hpp"
@@ -110,6 +111,8 @@ struct ddm_engine {
     long long pieces = 0;
     int R = 0, jmax = 32;
     float2 *ring = nullptr, *acc = nullptr, *tw = nullptr;
+    float2 *fft_mid = nullptr;  // output of the FFT row pass, fft_mid_frames frames (0: in place in the ring)
+    int fft_mid_frames = 0;
     // split-BF16 tensor-core DFT of the tiles of side 32, 64, 128 (ddm_config.small_tile_dft):
     // its cos/sin tables per log2 s - 5, in the kernel's shared-memory layout
     bool small_dft = false;
@@ -159,6 +162,9 @@ struct ddm_engine {
     long long wait_cycles = kWaitCycles;    // limit of every lag-pipeline wait (ddm_set_wait_limit)
     int inject = DDM_FAULT_NONE;            // one-shot fault for the next lag launch (ddm_inject_fault)
     LagMaps maps;                           // 2-D tensor maps of the ring for the lag kernel
+    HistShape hist;                         // CTA shape of the resident-history lag kernel (EB 0: not used)
+    RingLayout lay;                         // where a ring slot's elements live
+    AccLayout acc_lay;                      // and the accumulators
     bool defer_lag = false;                 // served: lag launches are collected, not issued
     std::vector<DeferredLag> deferred;
     size_t device_bytes = 0;
@@ -225,7 +231,7 @@ int dev_alloc(ddm_engine *e, Tp **p, size_t count) {
 void free_all(ddm_engine *e) {
     if (e->upload_stream) cudaStreamSynchronize(e->upload_stream);  // uploads read pinned buffers freed below
     if (e->stream && e->ev_isf_read) cudaStreamWaitEvent(e->stream, e->ev_isf_read, 0);  // a result copy reads isf_d
-    void *dev[] = {e->ring, e->acc, e->tw, e->stage, e->tables_d, e->chunk_beg_d, e->chunk_end_d,
+    void *dev[] = {e->ring, e->acc, e->tw, e->fft_mid, e->stage, e->tables_d, e->chunk_beg_d, e->chunk_end_d,
                    e->chunk_first_d, e->chunk_count_d, e->partial_d, e->idx_d, e->counts_d, e->norm_d,
                    e->isf_d, e->fit_d, e->status_d, e->dft_tab[0], e->dft_tab[1], e->dft_tab[2]};
     cudaStream_t fs = e->stream ? e->stream : e->fft_stream;
@@ -329,9 +335,9 @@ int launch_fft(ddm_engine *e, const uint8_t *src, long long frame_stride, long l
                     ? 1
                     : 0;
     rows.ring = e->ring;
-    rows.E = e->E;
-    rows.R = e->R;
+    rows.lay = e->lay;
     rows.tw = e->tw;
+    rows.mid = e->fft_mid;
     cols = rows;
     std::vector<FftScale> tile_scales;  // scales of side 32..128 through the per-tile kernel
     int row_ctas = 0, col_ctas = 0, nfft = 0;
@@ -375,9 +381,10 @@ int launch_fft(ddm_engine *e, const uint8_t *src, long long frame_stride, long l
     // 0.98 / 1 / 1.015 / 1.025), and two or more groups per piece keep the host copies of a
     // group overlapping the FFT of the one before (one group per piece: -6 % end to end).
     const long long frame_bytes = e->E * static_cast<long long>(sizeof(float2));
-    const int group = e->fft_group > 0 ? std::min(e->fft_group, nframes)
-                                       : static_cast<int>(std::max<long long>(
-                                             1, std::min<long long>(nframes, (256LL << 20) / frame_bytes)));
+    int group = e->fft_group > 0 ? std::min(e->fft_group, nframes)
+                                 : static_cast<int>(std::max<long long>(
+                                       1, std::min<long long>(nframes, (256LL << 20) / frame_bytes)));
+    if (e->fft_mid_frames > 0) group = std::min(group, e->fft_mid_frames);
     for (int f0 = 0; f0 < nframes; f0 += group) {
         const int nf = std::min(group, nframes - f0);
         if (before_group) {
@@ -419,9 +426,8 @@ int launch_fft(ddm_engine *e, const uint8_t *src, long long frame_stride, long l
             d.x_off = x_off;
             d.y_off = y_off;
             d.ring = e->ring;
-            d.E = e->E;
+            d.lay = e->lay;
             d.first_label = first_label + f0;
-            d.R = e->R;
             d.nframes = nf;
             d.sc = fs;
             d.tables = e->dft_tab[fs.log2s - kDftMinLog2];
@@ -467,27 +473,10 @@ int lag_resident_ctas(ddm_engine *e, int key, size_t smem, K kernel, int threads
     return n;
 }
 
-int launch_lag(ddm_engine *e, const Launch &L) {
-    if (L.nreg <= 0 || L.ent_acc.empty()) return DDM_OK;
-    const int J = lag_pick_j(L.nreg);
-    if (J == 0) return fail(DDM_ERR_STATE, "internal: no lag kernel for this frame count");
-    std::vector<int> table;
-    std::string err = build_lag_table(L.nreg, L.reg, L.ent_acc, L.ent_w, L.pos, J, &table);
-    if (!err.empty()) return fail(DDM_ERR_STATE, "internal: " + err);
+// Copies a table to the next device table slot, ordered before the engine's next lag launch.
+int upload_table(ddm_engine *e, const std::vector<int> &table, int *slot, int **device) {
     const int ntab = static_cast<int>(table.size());
     if (ntab > e->tab_stride) return fail(DDM_ERR_STATE, "internal: lag table overflow");
-    if (e->inject == DDM_FAULT_LAG_WAIT) {
-        // Test of the error path: the last entry's window is moved to start at the end of
-        // the partner list, so it reaches groups the producer never issues and the
-        // consumers' waits run out. Every entry becomes a single full window (no fused
-        // runs, no per-slot checks), so every shared-memory offset stays masked to the ring
-        // and the kernel reads nothing outside its table.
-        int *ent_ub = table.data() + kTabEntries + L.ent_acc.size();
-        int *ent_full = ent_ub + L.ent_acc.size();
-        for (size_t i = 0; i < L.ent_acc.size(); i++) ent_full[i] = kLagFullFlag;
-        ent_ub[L.ent_acc.size() - 1] = table[kTabNgroups] * kLagGroup;
-        e->inject = DDM_FAULT_NONE;
-    }
     const int ts = e->tab_next;
     e->tab_next = (e->tab_next + 1) % kTables;
     if (e->tab_used[ts]) CUDA_TRY(cudaEventSynchronize(e->tab_ev[ts]));
@@ -504,12 +493,125 @@ int launch_lag(ddm_engine *e, const Launch &L) {
         CUDA_TRY(cudaStreamWaitEvent(e->stream, e->tab_ev[ts], 0));
     }
     e->tab_used[ts] = true;
+    *slot = ts;
+    *device = td;
+    return DDM_OK;
+}
+
+// Shared-memory limits of the instances an engine's lag launches can use.
+cudaError_t set_lag_limits(const HistShape &shape) {
+    cudaError_t err = cudaSuccess;
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+#define HIST_ATTR(JJ, BB, WW)                                       \
+    if (err == cudaSuccess && shape.EB == BB && shape.CW == WW)      \
+        err = cudaFuncSetAttribute(lag_hist_kernel<JJ, BB, WW>, attr, kHistSmemMax);
+    HIST_INSTANCES(HIST_ATTR)
+#undef HIST_ATTR
+#define LAG_ATTR(JJ, GG) \
+    if (err == cudaSuccess && shape.EB == 0) err = cudaFuncSetAttribute(lag_pipe_kernel<JJ, GG>, attr, kLagSmemMax);
+    LAG_ATTR(4, 0) LAG_ATTR(8, 0) LAG_ATTR(16, 0) LAG_ATTR(20, 0) LAG_ATTR(24, 0) LAG_ATTR(30, 0) LAG_ATTR(32, 0)
+    LAG_ATTR(64, 0)
+    LAG_ATTR(4, 1) LAG_ATTR(8, 1) LAG_ATTR(16, 1) LAG_ATTR(20, 1) LAG_ATTR(24, 1) LAG_ATTR(30, 1) LAG_ATTR(32, 1)
+#undef LAG_ATTR
+    return err;
+}
+
+// CTAs for `blocks` units of work with `resident` CTAs at once: as few as finish in the same number
+// of rounds, so that a small launch leaves SMs to the next piece's FFT.
+unsigned balanced_grid(unsigned blocks, unsigned resident) {
+    if (blocks <= resident) return blocks;
+    const unsigned rounds = (blocks + resident - 1) / resident;
+    return (blocks + rounds - 1) / rounds;
+}
+
+// Queues the launch on the resident-history kernel.
+int launch_hist(ddm_engine *e, const Launch &L) {
+    HistInput in;
+    in.nreg = L.nreg;
+    in.reg.assign(L.reg, L.reg + L.nreg);
+    in.ent_acc = L.ent_acc;
+    in.ent_w = L.ent_w;
+    in.pos = L.pos;
+    HistTable table;
+    const int EB = e->hist.EB, CW = e->hist.CW;
+    std::string err = build_hist_table(in, e->hist, &table);
+    if (!err.empty()) return fail(DDM_ERR_STATE, "internal: " + err);
+    if (table.steps == 0 && e->inject == DDM_FAULT_NONE) return DDM_OK;  // no frame has a partner yet
+    if (e->inject == DDM_FAULT_LAG_WAIT) {
+        // Test of the error path: the first sub-batch's barrier expects one arrival more than the
+        // producer makes, so the consumers' waits run out. Nothing else changes.
+        table.ints[kHtArrive]++;
+        e->inject = DDM_FAULT_NONE;
+    }
+    int ts = -1, *td = nullptr;
+    HistInline inl;
+    if (!e->defer_lag && table.ints.size() <= kHistInlineInts) {
+        std::copy(table.ints.begin(), table.ints.end(), inl.v);
+    } else {
+        int st = upload_table(e, table.ints, &ts, &td);
+        if (st) return st;
+    }
+    const int J = hist_pick_j(L.nreg);
+    const unsigned blocks = static_cast<unsigned>((e->lay.E + EB - 1) / EB);
+    if (e->defer_lag) {  // a server issues it with other engines' work in one launch
+        e->deferred.push_back(DeferredLag{J, EB, CW, td, blocks, table.smem});
+        return DDM_OK;
+    }
+    const HistTarget target{e->ring, e->acc, e->lay, e->T, e->status_d, e->wait_cycles};
+    TimedRange tr(e, 1);
+    switch (hist_key(J, EB, CW)) {
+#define HIST_CASE(JJ, BB, WW)                                                                                     \
+    case hist_key(JJ, BB, WW): {                                                                                  \
+        const int per_sm = lag_resident_ctas(e, (1 << 20) + hist_key(JJ, BB, WW), table.smem,                    \
+                                             lag_hist_kernel<JJ, BB, WW>, hist_threads(WW));                     \
+        const unsigned grid = balanced_grid(blocks, static_cast<unsigned>(per_sm * e->sms));                     \
+        lag_hist_kernel<JJ, BB, WW><<<grid, hist_threads(WW), table.smem, e->stream>>>(                           \
+            target, td, static_cast<int>(blocks), inl);                                                           \
+        break;                                                                                                    \
+    }
+        HIST_INSTANCES(HIST_CASE)
+#undef HIST_CASE
+        default: return fail(DDM_ERR_STATE, "internal: no lag kernel for this frame count");
+    }
+    CUDA_TRY(cudaGetLastError());
+    if (ts >= 0) CUDA_TRY(cudaEventRecord(e->tab_free[ts], e->stream));
+    tr.end(1);
+    e->launches++;
+    // every distinct frame read once, every accumulator row read and written once
+    e->tbytes[1] += 8.0 * static_cast<double>(e->E) * (table.frames + 2.0 * L.ent_acc.size());
+    return DDM_OK;
+}
+
+int launch_lag(ddm_engine *e, const Launch &L) {
+    if (L.nreg <= 0 || L.ent_acc.empty()) return DDM_OK;
+    if (e->hist.EB) return launch_hist(e, L);
+    const int J = lag_pick_j(L.nreg);
+    if (J == 0) return fail(DDM_ERR_STATE, "internal: no lag kernel for this frame count");
+    std::vector<int> table;
+    std::string err = build_lag_table(L.nreg, L.reg, L.ent_acc, L.ent_w, L.pos, J, &table);
+    if (!err.empty()) return fail(DDM_ERR_STATE, "internal: " + err);
+    const int ntab = static_cast<int>(table.size());
+    if (e->inject == DDM_FAULT_LAG_WAIT) {
+        // Test of the error path: the last entry's window is moved to start at the end of
+        // the partner list, so it reaches groups the producer never issues and the
+        // consumers' waits run out. Every entry becomes a single full window (no fused
+        // runs, no per-slot checks), so every shared-memory offset stays masked to the ring
+        // and the kernel reads nothing outside its table.
+        int *ent_ub = table.data() + kTabEntries + L.ent_acc.size();
+        int *ent_full = ent_ub + L.ent_acc.size();
+        for (size_t i = 0; i < L.ent_acc.size(); i++) ent_full[i] = kLagFullFlag;
+        ent_ub[L.ent_acc.size() - 1] = table[kTabNgroups] * kLagGroup;
+        e->inject = DDM_FAULT_NONE;
+    }
+    int ts, *td;
+    int st = upload_table(e, table, &ts, &td);
+    if (st) return st;
 
     const int G = J <= 32 ? e->lag_geom : 0;
     const unsigned blocks = static_cast<unsigned>((e->E + lag_cta_elems(J, G) - 1) / lag_cta_elems(J, G));
     const size_t smem = lag_smem_bytes(J, ntab, G);
     if (e->defer_lag) {  // a server issues it with other engines' work in one launch
-        e->deferred.push_back(DeferredLag{J, td, blocks, smem});
+        e->deferred.push_back(DeferredLag{J, 0, 0, td, blocks, smem});
         return DDM_OK;
     }
     TimedRange tr(e, 1);
@@ -624,19 +726,27 @@ int lag_iteration(ddm_engine *e, const CompatIteration &it) {
 
 int run_azimuth(ddm_engine *e, const std::vector<double> &norm) {
     CUDA_TRY(cudaStreamWaitEvent(e->stream, e->ev_isf_read, 0));  // a result copy may still read isf_d
-    // the upload reads its pinned half asynchronously: refill a half only once its previous
-    // upload (two finalizes ago) has run; the upload into the device half waits for the
-    // azimuthal average that last read it
-    const int ns = e->norm_slot;
-    e->norm_slot ^= 1;
-    double *nh = e->norm_h + static_cast<size_t>(ns) * e->T;
-    double *nd = e->norm_d + static_cast<size_t>(ns) * e->T;
-    CUDA_TRY(cudaEventSynchronize(e->norm_ev[ns]));
-    std::copy(norm.begin(), norm.end(), nh);
-    CUDA_TRY(cudaStreamWaitEvent(e->upload_stream, e->norm_free[ns], 0));
-    CUDA_TRY(cudaMemcpyAsync(nd, nh, sizeof(double) * e->T, cudaMemcpyHostToDevice, e->upload_stream));
-    CUDA_TRY(cudaEventRecord(e->norm_ev[ns], e->upload_stream));
-    CUDA_TRY(cudaStreamWaitEvent(e->stream, e->norm_ev[ns], 0));
+    AzNorm inl;
+    const bool inline_norm = e->T <= kAzInlineNorms;
+    double *nd = nullptr;
+    int ns = 0;
+    if (inline_norm) {
+        std::copy(norm.begin(), norm.end(), inl.v);
+    } else {
+        // the upload reads its pinned half asynchronously: refill a half only once its previous
+        // upload (two finalizes ago) has run; the upload into the device half waits for the
+        // azimuthal average that last read it
+        ns = e->norm_slot;
+        e->norm_slot ^= 1;
+        double *nh = e->norm_h + static_cast<size_t>(ns) * e->T;
+        nd = e->norm_d + static_cast<size_t>(ns) * e->T;
+        CUDA_TRY(cudaEventSynchronize(e->norm_ev[ns]));
+        std::copy(norm.begin(), norm.end(), nh);
+        CUDA_TRY(cudaStreamWaitEvent(e->upload_stream, e->norm_free[ns], 0));
+        CUDA_TRY(cudaMemcpyAsync(nd, nh, sizeof(double) * e->T, cudaMemcpyHostToDevice, e->upload_stream));
+        CUDA_TRY(cudaEventRecord(e->norm_ev[ns], e->upload_stream));
+        CUDA_TRY(cudaStreamWaitEvent(e->stream, e->norm_ev[ns], 0));
+    }
     e->host_norm = norm;
     AzArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -645,7 +755,7 @@ int run_azimuth(ddm_engine *e, const std::vector<double> &norm) {
     a.Q = e->Q;
     for (int s = 0; s < e->S; s++) a.sc[s] = e->sd[s];
     a.acc = e->acc;
-    a.E = e->E;
+    a.lay = e->acc_lay;
     a.idx = e->idx_d;
     a.chunk_beg = e->chunk_beg_d;
     a.chunk_end = e->chunk_end_d;
@@ -663,9 +773,10 @@ int run_azimuth(ddm_engine *e, const std::vector<double> &norm) {
                                  e->stream>>>(a);
         CUDA_TRY(cudaGetLastError());
     }
-    azimuth_final_kernel<<<static_cast<unsigned>((a.bins + kAzThreads - 1) / kAzThreads), kAzThreads, 0, e->stream>>>(a);
+    azimuth_final_kernel<<<static_cast<unsigned>((a.bins + kAzThreads - 1) / kAzThreads), kAzThreads, 0, e->stream>>>(a,
+                                                                                                                inl);
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaEventRecord(e->norm_free[ns], e->stream));
+    if (!inline_norm) CUDA_TRY(cudaEventRecord(e->norm_free[ns], e->stream));
     tr.end(a.items > 0 ? 2 : 1);
     e->tbytes[2] += e->az_bytes;
     e->launches += a.items > 0 ? 2 : 1;
@@ -673,7 +784,7 @@ int run_azimuth(ddm_engine *e, const std::vector<double> &norm) {
 }
 
 int purge(ddm_engine *e) {
-    CUDA_TRY(cudaMemsetAsync(e->acc, 0, sizeof(float2) * e->T * e->E, e->stream));
+    CUDA_TRY(cudaMemsetAsync(e->acc, 0, sizeof(float2) * e->T * e->lay.E, e->stream));
     std::fill(e->pair_count.begin(), e->pair_count.end(), 0.0);
     return DDM_OK;
 }
@@ -895,14 +1006,53 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
         cudaEventCreateWithFlags(&e->ev_guard[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&e->ev_guard[1], cudaEventDisableTiming) != cudaSuccess)
         return bail(fail(DDM_ERR_CUDA, "stream/event creation failed"));
+    // Launches of up to 32 frames of geometry 0 run on the resident-history kernel where their
+    // frames fit its shared memory, on a ring in slabs; the ring kernel keeps the others.
+    if (e->lag_geom == 0 && e->lag_batch <= kHistMaxJ) {
+        HistInput steady;
+        steady.nreg = e->lag_batch;
+        for (int p = 0; p < e->tau_max + e->lag_batch; p++) steady.pos.push_back(p % e->R);
+        for (int i = 0; i < e->T; i++) {
+            steady.ent_acc.push_back(i);
+            steady.ent_w.push_back(compat ? e->taus[i] : e->tau_max - e->taus[e->T - 1 - i]);
+        }
+        const int first = compat ? 0 : e->tau_max;
+        steady.reg.assign(steady.pos.begin() + first, steady.pos.begin() + first + e->lag_batch);
+        e->hist = hist_pick_shape(steady);
+        if (e->hist.EB)
+            e->tab_stride = std::max(e->tab_stride, hist_table_capacity(e->T, e->tau_max + e->lag_batch, 1));
+    }
+    if (e->hist.EB) {
+        e->lay = RingLayout{(e->E + 15) / 16 * 16, e->R, 1};
+        e->acc_lay = AccLayout{16, 16LL * e->T};
+    } else {
+        e->lay = RingLayout{e->E, e->R, 0};
+        e->acc_lay = AccLayout{e->E, 16};
+    }
     int st;
-    if ((st = dev_alloc(e, &e->ring, static_cast<size_t>(e->R) * e->E))) return bail(st);
-    {
+    if ((st = dev_alloc(e, &e->ring, static_cast<size_t>(e->R) * e->lay.E))) return bail(st);
+    if (!e->hist.EB) {
         std::string err = make_lag_maps(e->ring, e->E, e->R, &e->maps);
         if (!err.empty()) return bail(fail(DDM_ERR_CUDA, err));
     }
-    if ((st = dev_alloc(e, &e->acc, static_cast<size_t>(e->T) * e->E))) return bail(st);
+    if ((st = dev_alloc(e, &e->acc, static_cast<size_t>(e->T) * e->lay.E))) return bail(st);
     if ((st = dev_alloc(e, &e->stage, stage_bytes))) return bail(st);
+    if (e->lay.slabs) {
+        // The row pass's output of one FFT group, in frame order: at most 256 MB. Not part of the budget
+        // check: left out where it does not fit.
+        const size_t frame = sizeof(float2) * e->lay.E;
+        const int frames = static_cast<int>(std::min<size_t>(e->jmax, (256u << 20) / frame));
+        const size_t bytes = frame * frames;
+        if (frames > 0 && (!cfg->hbm_budget_bytes || need + bytes <= cfg->hbm_budget_bytes)) {
+            if (dev_alloc(e, &e->fft_mid, static_cast<size_t>(frames) * e->lay.E) == DDM_OK) {
+                e->fft_mid_frames = frames;
+            } else {
+                e->fft_mid = nullptr;
+                cudaGetLastError();
+                clear_error();
+            }
+        }
+    }
     if ((st = dev_alloc(e, &e->tables_d, static_cast<size_t>(kTables) * e->tab_stride))) return bail(st);
     if ((st = dev_alloc(e, &e->norm_d, 2 * e->T))) return bail(st);
     if ((st = dev_alloc(e, &e->isf_d, e->isf_size))) return bail(st);
@@ -952,9 +1102,17 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
     {
         std::vector<int> idx_all, cbeg, cend, cfirst, ccount;
         long long items = 0;
+        std::vector<std::vector<int>> qps(e->S), idxs(e->S), countss(e->S);
+        long long warps = 0;
         for (int s = 0; s < e->S; s++) {
-            std::vector<int> qp, idx, counts;
-            build_masks(e->scales[s], e->lambdas, e->tol, &qp, &idx, &counts);
+            build_masks(e->scales[s], e->lambdas, e->tol, &qps[s], &idxs[s], &countss[s]);
+            for (int q = 0; q < e->Q; q++)
+                warps += static_cast<long long>(e->sd[s].tiles) * e->T * ((countss[s][q] + kAzChunk - 1) / kAzChunk);
+        }
+        int chunk = kAzChunk;
+        for (; chunk > kAzMinChunk && warps < kAzWantWarps; warps *= 2) chunk /= 2;
+        for (int s = 0; s < e->S; s++) {
+            std::vector<int> &qp = qps[s], &idx = idxs[s], &counts = countss[s];
             const int base = static_cast<int>(idx_all.size());
             ScaleDesc &d = e->sd[s];
             d.chunk_off = static_cast<int>(cbeg.size());
@@ -962,9 +1120,9 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
             for (int q = 0; q < e->Q; q++) {
                 cfirst.push_back(nloc);
                 int n = 0;
-                for (int b = qp[q]; b < qp[q + 1]; b += kAzChunk, n++) {
+                for (int b = qp[q]; b < qp[q + 1]; b += chunk, n++) {
                     cbeg.push_back(base + b);
-                    cend.push_back(base + std::min(b + kAzChunk, qp[q + 1]));
+                    cend.push_back(base + std::min(b + chunk, qp[q + 1]));
                 }
                 ccount.push_back(n);
                 nloc += n;
@@ -1002,21 +1160,7 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
         cudaFuncSetAttribute(fft_tile_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(fft_tile_smem_bytes(128))) != cudaSuccess ||
         cudaFuncSetAttribute(fft_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<20>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<30>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<20, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<24, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<30, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(lag_pipe_kernel<32, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLagSmemMax) != cudaSuccess ||
+        set_lag_limits(e->hist) != cudaSuccess ||
         cudaFuncSetAttribute(dft_bf16_kernel<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft_smem_bytes(32)) != cudaSuccess ||
         cudaFuncSetAttribute(dft_bf16_kernel<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft_smem_bytes(64)) != cudaSuccess ||
         cudaFuncSetAttribute(dft_bf16_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft_smem_bytes(128)) != cudaSuccess)
@@ -1027,8 +1171,8 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
     // server's shared stream stays free while a new stream is set up). The unbiased
     // estimator never reads a ring slot before its frame is written, so only compat mode
     // (whose reference schedule can name frames it never wrote) clears the ring.
-    if (cudaMemsetAsync(e->acc, 0, acc_bytes, e->fft_stream) != cudaSuccess ||
-        (compat && cudaMemsetAsync(e->ring, 0, ring_bytes, e->fft_stream) != cudaSuccess) ||
+    if (cudaMemsetAsync(e->acc, 0, sizeof(float2) * e->T * e->lay.E, e->fft_stream) != cudaSuccess ||
+        (compat && cudaMemsetAsync(e->ring, 0, sizeof(float2) * e->R * e->lay.E, e->fft_stream) != cudaSuccess) ||
         (e->own_stream && cudaStreamSynchronize(e->fft_stream) != cudaSuccess))
         return bail(fail(DDM_ERR_CUDA, "initial memset failed"));
     *out = e;
@@ -1187,6 +1331,10 @@ std::vector<DeferredLag> engine_take_deferred(ddm_engine *e) {
 
 LagTarget engine_lag_target(const ddm_engine *e) { return LagTarget{e->ring, e->acc, e->E, e->status_d, &e->maps}; }
 
+HistTarget engine_hist_target(const ddm_engine *e) {
+    return HistTarget{e->ring, e->acc, e->lay, e->T, e->status_d, e->wait_cycles};
+}
+
 cudaStream_t engine_stream(const ddm_engine *e) { return e->stream; }
 const double *engine_isf_device(const ddm_engine *e) { return e->isf_d; }
 const int *engine_status_device(const ddm_engine *e) { return e->status_d; }
@@ -1333,8 +1481,38 @@ extern "C" int ddm_read_spectrum(ddm_engine *e, int frame, float *out, long capa
         return fail(DDM_ERR_INVALID_ARG, "frame is not in the ring");
     CUDA_TRY(cudaStreamSynchronize(e->fft_stream));
     CUDA_TRY(cudaStreamSynchronize(e->stream));
-    CUDA_TRY(cudaMemcpy(out, e->ring + static_cast<size_t>(frame % e->R) * e->E, sizeof(float2) * e->E,
-                        cudaMemcpyDeviceToHost));
+    const int slot = static_cast<int>(frame % e->R);
+    const float2 *src = e->ring + e->lay.base(slot);
+    const size_t bytes = sizeof(float2) * e->E;
+    float2 *packed = nullptr;
+    if (e->lay.slabs && cudaMallocAsync(reinterpret_cast<void **>(&packed), bytes, e->stream) != cudaSuccess) {
+        cudaGetLastError();  // no room to gather the frame on the device: block by block
+        const size_t whole = static_cast<size_t>(e->E / 16);
+        CUDA_TRY(cudaMemcpy2D(out, 128, src, sizeof(float2) * e->lay.stride(slot), 128, whole, cudaMemcpyDeviceToHost));
+        CUDA_TRY(cudaMemcpy(out + whole * 32, src + whole * e->lay.stride(slot), bytes - whole * 128,
+                            cudaMemcpyDeviceToHost));
+        return DDM_OK;
+    }
+    cudaError_t err = cudaSuccess;
+    if (packed) {
+        gather_frame_kernel<<<static_cast<unsigned>((e->E + 255) / 256), 256, 0, e->stream>>>(src, e->lay.stride(slot),
+                                                                                              packed, e->E);
+        err = cudaGetLastError();
+        if (err == cudaSuccess) err = cudaStreamSynchronize(e->stream);
+        src = packed;
+    }
+    if (err == cudaSuccess) err = cudaMemcpy(out, src, bytes, cudaMemcpyDeviceToHost);
+    if (packed) cudaFreeAsync(packed, e->stream);
+    CUDA_TRY(err);
+    return DDM_OK;
+}
+
+// The accumulators as the device lays them out, in host memory.
+static int copy_accumulators(ddm_engine *e, std::vector<float2> *host) {
+    host->resize(static_cast<size_t>(e->T) * e->lay.E);
+    CUDA_TRY(cudaStreamSynchronize(e->fft_stream));
+    CUDA_TRY(cudaStreamSynchronize(e->stream));
+    CUDA_TRY(cudaMemcpy(host->data(), e->acc, sizeof(float2) * host->size(), cudaMemcpyDeviceToHost));
     return DDM_OK;
 }
 
@@ -1343,11 +1521,13 @@ extern "C" int ddm_read_accumulators(ddm_engine *e, double *out, long capacity) 
     if (!e || !out || capacity < static_cast<long>(e->T * e->E)) return fail(DDM_ERR_INVALID_ARG, "bad argument");
     int st = flush_lag(e);
     if (st) return st;
-    std::vector<float2> tmp(static_cast<size_t>(e->T) * e->E);
-    CUDA_TRY(cudaStreamSynchronize(e->fft_stream));
-    CUDA_TRY(cudaStreamSynchronize(e->stream));
-    CUDA_TRY(cudaMemcpy(tmp.data(), e->acc, sizeof(float2) * tmp.size(), cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < tmp.size(); i++) out[i] = static_cast<double>(tmp[i].x) - static_cast<double>(tmp[i].y);
+    std::vector<float2> tmp;
+    if ((st = copy_accumulators(e, &tmp))) return st;
+    for (int t = 0; t < e->T; t++)
+        for (long long k = 0; k < e->E; k++) {
+            const float2 v = tmp[e->acc_lay.at(t, k)];
+            out[t * e->E + k] = static_cast<double>(v.x) - static_cast<double>(v.y);
+        }
     return DDM_OK;
 }
 
@@ -1374,16 +1554,18 @@ extern "C" int ddm_read_unaveraged(ddm_engine *e, double *out, long capacity) {
     if (!e || !out || capacity < static_cast<long>(e->T * e->E))
         return fail(DDM_ERR_INVALID_ARG, "ddm_read_unaveraged: bad argument");
     if (!e->finalized) return fail(DDM_ERR_STATE, "ddm_finalize has not run");
-    std::vector<float2> tmp(static_cast<size_t>(e->T) * e->E);
-    CUDA_TRY(cudaStreamSynchronize(e->stream));
-    CUDA_TRY(cudaMemcpy(tmp.data(), e->acc, sizeof(float2) * tmp.size(), cudaMemcpyDeviceToHost));
+    std::vector<float2> tmp;
+    int st = copy_accumulators(e, &tmp);
+    if (st) return st;
     for (int t = 0; t < e->T; t++) {
         const double nrm = e->host_norm[t];
         for (const ScaleDesc &d : e->sd) {
             const double f = nrm != 0.0 ? 2.0 * d.inv_s4 / nrm : 0.0;
-            const size_t b = static_cast<size_t>(t) * e->E + d.off, n = static_cast<size_t>(d.tiles) * d.n;
-            for (size_t k = b; k < b + n; k++)
-                out[k] = (static_cast<double>(tmp[k].x) - static_cast<double>(tmp[k].y)) * f;
+            const long long end = d.off + d.tiles * d.n;
+            for (long long k = d.off; k < end; k++) {
+                const float2 v = tmp[e->acc_lay.at(t, k)];
+                out[t * e->E + k] = (static_cast<double>(v.x) - static_cast<double>(v.y)) * f;
+            }
         }
     }
     return DDM_OK;

@@ -8,6 +8,7 @@
 
 #include "../../include/ddm.h"
 #include "lag.cuh"
+#include "lag_hist.cuh"
 
 namespace ddm {
 
@@ -17,6 +18,7 @@ constexpr int kEngineStreams = 4;
 
 struct DeferredLag {  // one lag launch an engine would have issued
     int J;
+    int EB, CW;        // resident-history kernel: its CTA shape; 0: the ring kernel
     const int *table;  // device copy of its table (the engine's table ring)
     unsigned blocks;
     size_t smem;
@@ -35,6 +37,7 @@ struct LagTarget {  // what a lag launch of this engine reads and writes
 void engine_defer_lag(ddm_engine *e, bool on);
 std::vector<DeferredLag> engine_take_deferred(ddm_engine *e);
 LagTarget engine_lag_target(const ddm_engine *e);
+HistTarget engine_hist_target(const ddm_engine *e);
 // Validation and sizing of ddm_open only: the device bytes checked against the HBM budget.
 int engine_plan_bytes(const ddm_config *cfg, size_t *need);
 // ddm_close without synchronising: device memory is freed in stream order on the engine's

@@ -113,9 +113,8 @@ inline int lag_pick_j(int nreg) {
     return 0;
 }
 
-// Tensor maps of a ring float2[slots][E] for boxes of 128 or 64 elements (the element blocks
-// of the one- and two-lane kernels) x 1, 2, 4, 8 slots.
-inline std::string make_lag_maps(const void *ring, long long E, int slots, LagMaps *maps) {
+// One tensor map of a ring float2[slots][E]: boxes of `width` elements x `rows` slots.
+inline std::string encode_ring_map(CUtensorMap *map, const void *ring, long long E, int slots, int width, int rows) {
     // looked up once, by a thread-safe static initialiser (engines on several threads and
     // the static entry point all come through here)
     static const PFN_cuTensorMapEncodeTiled_v12000 encode = []() -> PFN_cuTensorMapEncodeTiled_v12000 {
@@ -132,17 +131,23 @@ inline std::string make_lag_maps(const void *ring, long long E, int slots, LagMa
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(E), static_cast<cuuint64_t>(slots)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(E) * 8};
     const cuuint32_t estr[2] = {1, 1};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(width), static_cast<cuuint32_t>(rows)};
+    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<void *>(ring), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r));
+    return std::string();
+}
+
+// Tensor maps of a ring float2[slots][E] for boxes of 128 or 64 elements (the element blocks
+// of the one- and two-lane kernels) x 1, 2, 4, 8 slots.
+inline std::string make_lag_maps(const void *ring, long long E, int slots, LagMaps *maps) {
     const int widths[2] = {lag_cta_elems(1), lag_cta_elems(kLagMaxJ)};
-    for (int w = 0; w < 2; w++) {
+    for (int w = 0; w < 2; w++)
         for (int k = 0; k < kLagRunKinds; k++) {
-            const cuuint32_t box[2] = {static_cast<cuuint32_t>(widths[w]), 1u << k};
-            CUresult r = encode(&maps->box[w][k], CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<void *>(ring), dims,
-                                strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS)
-                return "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r));
+            std::string err = encode_ring_map(&maps->box[w][k], ring, E, slots, widths[w], 1 << k);
+            if (!err.empty()) return err;
         }
-    }
     return std::string();
 }
 

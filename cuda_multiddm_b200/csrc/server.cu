@@ -24,6 +24,7 @@
 #include "engine_internal.hpp"
 #include "errors.hpp"
 #include "lag.cuh"
+#include "lag_hist.cuh"
 #include "pinned_pool.hpp"
 #include "stream_pool.hpp"
 
@@ -75,6 +76,11 @@ struct Stream {
     std::vector<PinnedBuf> free_bufs;
 };
 
+union BatchItem {  // a descriptor of either batched lag kernel
+    LagBatchItem lag;
+    HistBatchItem hist;
+};
+
 void CUDART_CB on_result(void *arg) {  // runs on a CUDA driver thread: no CUDA calls here
     Slot *s = static_cast<Slot *>(arg);
     s->done_s.store(ddm_server_clock(s->server));
@@ -84,7 +90,7 @@ void CUDART_CB on_result(void *arg) {  // runs on a CUDA driver thread: no CUDA 
 }  // namespace
 
 struct ddm_server {
-    int device = 0;
+    int device = 0, sms = 0;
     cudaStream_t stream = nullptr;
     size_t budget = 0, used = 0, reserved = 0;
     int opening = 0;  // streams being admitted outside the lock
@@ -95,7 +101,7 @@ struct ddm_server {
     std::list<Stream> closing;  // removed, waiting for their queued work before release
     mutable std::mutex lock;
     // batched lag descriptors
-    LagBatchItem *items_h = nullptr, *items_d = nullptr;
+    BatchItem *items_h = nullptr, *items_d = nullptr;
     int items_cap = 0, items_next = 0;
     cudaEvent_t items_ev[kItemRing] = {};
     bool items_used[kItemRing] = {};
@@ -192,42 +198,68 @@ int ensure_items(ddm_server *s, int n) {
     s->items_h = nullptr;
     s->items_d = nullptr;
     const int cap = std::max(n, 64);
-    if (cudaMallocHost(reinterpret_cast<void **>(&s->items_h), sizeof(LagBatchItem) * cap * kItemRing) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void **>(&s->items_d), sizeof(LagBatchItem) * cap * kItemRing) != cudaSuccess)
+    if (cudaMallocHost(reinterpret_cast<void **>(&s->items_h), sizeof(BatchItem) * cap * kItemRing) != cudaSuccess ||
+        cudaMalloc(reinterpret_cast<void **>(&s->items_d), sizeof(BatchItem) * cap * kItemRing) != cudaSuccess)
         return fail(DDM_ERR_OUT_OF_MEMORY, "batch descriptor buffers");
     s->items_cap = cap;
     std::fill(s->items_used, s->items_used + kItemRing, false);
     return DDM_OK;
 }
 
-// One launch of lag_batch_kernel<J> over `work` (engine, its deferred launches of this J).
-int launch_batch(ddm_server *s, int J, const std::vector<std::pair<Stream *, DeferredLag>> &work) {
+// One launch of lag_batch_kernel<J> or lag_hist_batch_kernel<J, EB, CW> over `work` (engines, each
+// with one deferred launch of this kernel instance).
+int launch_batch(ddm_server *s, const std::vector<std::pair<Stream *, DeferredLag>> &work) {
     if (work.empty()) return DDM_OK;
     int st = ensure_items(s, static_cast<int>(work.size()));
     if (st) return st;
     const int ring = s->items_next;
     s->items_next = (s->items_next + 1) % kItemRing;
     if (s->items_used[ring]) CUDA_TRY(cudaEventSynchronize(s->items_ev[ring]));
-    LagBatchItem *h = s->items_h + static_cast<size_t>(ring) * s->items_cap;
-    LagBatchItem *d = s->items_d + static_cast<size_t>(ring) * s->items_cap;
-    int cta = 0;
-    size_t smem = 0;
-    for (size_t i = 0; i < work.size(); i++) {
-        const LagTarget t = engine_lag_target(work[i].first->eng);
-        h[i] = LagBatchItem{t.ring, t.acc, t.E, work[i].second.table, t.status, work[i].first->maps_d, cta, 0};
-        cta += static_cast<int>(work[i].second.blocks);
-        smem = std::max(smem, work[i].second.smem);
-    }
+    BatchItem *h = s->items_h + static_cast<size_t>(ring) * s->items_cap;
+    BatchItem *d = s->items_d + static_cast<size_t>(ring) * s->items_cap;
+    const int J = work[0].second.J, EB = work[0].second.EB, CW = work[0].second.CW;
     const int n = static_cast<int>(work.size());
-    CUDA_TRY(cudaMemcpyAsync(d, h, sizeof(LagBatchItem) * n, cudaMemcpyHostToDevice, s->stream));
+    size_t smem = 0;
+    long long blocks = 0;
+    for (const auto &w : work) {
+        smem = std::max(smem, w.second.smem);
+        blocks += w.second.blocks;
+    }
+    int cta = 0;
+    if (EB == 0) {
+        LagBatchItem *items = reinterpret_cast<LagBatchItem *>(h);
+        for (int i = 0; i < n; i++) {
+            const LagTarget t = engine_lag_target(work[i].first->eng);
+            items[i] = LagBatchItem{t.ring, t.acc, t.E, work[i].second.table, t.status, work[i].first->maps_d, cta, 0};
+            cta += static_cast<int>(work[i].second.blocks);
+        }
+    } else {
+        // a few CTAs per resident slot, so that the table and the barriers are set up once for many
+        // blocks and the items' ends still spread over the SMs
+        const long long per_cta = std::max<long long>(1, blocks / (4LL * hist_ctas_per_sm(CW) * s->sms));
+        HistBatchItem *items = reinterpret_cast<HistBatchItem *>(h);
+        for (int i = 0; i < n; i++) {
+            const int nb = static_cast<int>(work[i].second.blocks);
+            const int ctas = static_cast<int>((nb + per_cta - 1) / per_cta);
+            items[i] = HistBatchItem{engine_hist_target(work[i].first->eng), work[i].second.table, cta, ctas, nb};
+            cta += ctas;
+        }
+    }
+    CUDA_TRY(cudaMemcpyAsync(d, h, (EB ? sizeof(HistBatchItem) : sizeof(LagBatchItem)) * n, cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(cudaEventRecord(s->items_ev[ring], s->stream));
     s->items_used[ring] = true;
-    switch (J) {
+    switch (EB ? hist_key(J, EB, CW) : J) {
 #define BATCH_CASE(JJ) \
-    case JJ: lag_batch_kernel<JJ><<<cta, kLagThreads, smem, s->stream>>>(d, n); break;
+    case JJ: lag_batch_kernel<JJ><<<cta, kLagThreads, smem, s->stream>>>(reinterpret_cast<LagBatchItem *>(d), n); break;
         BATCH_CASE(4) BATCH_CASE(8) BATCH_CASE(16) BATCH_CASE(20) BATCH_CASE(24) BATCH_CASE(30) BATCH_CASE(32)
-        BATCH_CASE(64)
 #undef BATCH_CASE
+#define HIST_CASE(JJ, BB, WW)                                                                                  \
+    case hist_key(JJ, BB, WW):                                                                                 \
+        lag_hist_batch_kernel<JJ, BB, WW><<<cta, hist_threads(WW), smem, s->stream>>>(                         \
+            reinterpret_cast<HistBatchItem *>(d), n);                                                          \
+        break;
+        HIST_INSTANCES(HIST_CASE)
+#undef HIST_CASE
         default: return fail(DDM_ERR_STATE, "internal: no batched lag kernel for this frame count");
     }
     CUDA_TRY(cudaGetLastError());
@@ -251,6 +283,7 @@ extern "C" int ddm_server_open(const ddm_server_config *cfg, ddm_server **out) {
     std::unique_ptr<ddm_server> s(new ddm_server);
     s->device = cfg->device;
     if (cudaSetDevice(s->device) != cudaSuccess) return fail(DDM_ERR_NO_DEVICE, "cudaSetDevice failed");
+    CUDA_TRY(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device));
     size_t free_b = 0, total_b = 0;
     CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
     s->budget = cfg->hbm_budget_bytes ? cfg->hbm_budget_bytes : (free_b > (2ull << 30) ? free_b - (2ull << 30) : 0);
@@ -282,8 +315,12 @@ extern "C" int ddm_server_open(const ddm_server_config *cfg, ddm_server **out) {
     const int attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
 #define BATCH_ATTR(JJ) \
     CUDA_TRY(cudaFuncSetAttribute(lag_batch_kernel<JJ>, static_cast<cudaFuncAttribute>(attr), kLagSmemMax));
-    BATCH_ATTR(4) BATCH_ATTR(8) BATCH_ATTR(16) BATCH_ATTR(20) BATCH_ATTR(24) BATCH_ATTR(30) BATCH_ATTR(32) BATCH_ATTR(64)
+    BATCH_ATTR(4) BATCH_ATTR(8) BATCH_ATTR(16) BATCH_ATTR(20) BATCH_ATTR(24) BATCH_ATTR(30) BATCH_ATTR(32)
 #undef BATCH_ATTR
+#define HIST_ATTR(JJ, BB, WW) \
+    CUDA_TRY(cudaFuncSetAttribute(lag_hist_batch_kernel<JJ, BB, WW>, static_cast<cudaFuncAttribute>(attr), kHistSmemMax));
+    HIST_INSTANCES(HIST_ATTR)
+#undef HIST_ATTR
     *out = s.release();
     return DDM_OK;
 }
@@ -341,6 +378,7 @@ extern "C" int ddm_server_add_stream(ddm_server *s, const ddm_config *cfg, int *
             return fail(DDM_ERR_BUSY, "not admitted now: the stream needs " + std::to_string(need) +
                                           " device bytes, " + std::to_string(s->budget - s->used - s->reserved) +
                                           " of the budget are free");
+        c.hbm_budget_bytes = s->budget - s->used - s->reserved;  // for the engine's optional buffers
         s->reserved += need;
         s->opening++;
     }
@@ -466,7 +504,8 @@ extern "C" int ddm_server_step(ddm_server *s, int *chunks_issued) {
     for (auto &kv : s->streams) any = any || !kv.second.pending.empty();
     if (any && (ev0 = take_event(s))) CUDA_TRY(cudaEventRecord(ev0, s->stream));
     std::vector<std::pair<Stream *, Slot *>> taken;
-    std::map<int, std::vector<std::pair<Stream *, DeferredLag>>> by_j;
+    // by round and kernel instance: a stream's launches update the same accumulators one after another
+    std::map<std::pair<int, int>, std::vector<std::pair<Stream *, DeferredLag>>> rounds;
     // 1. each stream's next chunk: H2D copy and FFT (the engine's own stream pair), lag work deferred
     for (auto &kv : s->streams) {
         Stream &st = kv.second;
@@ -490,11 +529,13 @@ extern "C" int ddm_server_step(ddm_server *s, int *chunks_issued) {
         slot->state.store(1);
         st.order.push_back(slot);
         taken.emplace_back(&st, slot);
-        for (const DeferredLag &d : engine_take_deferred(st.eng)) by_j[d.J].emplace_back(&st, d);
+        int round = 0;
+        for (const DeferredLag &d : engine_take_deferred(st.eng))
+            rounds[{round++, d.EB ? hist_key(d.J, d.EB, d.CW) : d.J}].emplace_back(&st, d);
     }
-    // 2. one lag launch per register-frame count over every taken stream
-    for (auto &kv : by_j) {
-        int r = launch_batch(s, kv.first, kv.second);
+    // 2. one lag launch per kernel instance over every taken stream
+    for (auto &kv : rounds) {
+        int r = launch_batch(s, kv.second);
         if (r) return r;
     }
     // 3. per stream: azimuthal average, ISF and status to host, completion callback
