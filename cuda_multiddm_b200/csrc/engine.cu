@@ -1626,8 +1626,8 @@ extern "C" int ddm_fit_isf(ddm_engine *e, float fps, double um_per_px, int start
     CUDA_TRY(cudaMemcpyAsync(tau_d, host.data(), sizeof(double) * host.size(), cudaMemcpyHostToDevice, e->stream));
     fit_mean_kernel<<<static_cast<unsigned>((n_mean + kFitThreads - 1) / kFitThreads), kFitThreads, 0, e->stream>>>(a);
     CUDA_TRY(cudaGetLastError());
-    fit_isf_kernel<<<static_cast<unsigned>((tile_curves + scale_curves + kFitThreads - 1) / kFitThreads), kFitThreads,
-                     0, e->stream>>>(a);
+    fit_isf_kernel<<<static_cast<unsigned>((tile_curves + scale_curves + kFitWarps - 1) / kFitWarps), kFitThreads, 0,
+                     e->stream>>>(a);
     CUDA_TRY(cudaGetLastError());
     fit_diffusion_kernel<<<static_cast<unsigned>((tiles_total + e->S + kFitThreads - 1) / kFitThreads), kFitThreads, 0,
                            e->stream>>>(a, tiles_total);

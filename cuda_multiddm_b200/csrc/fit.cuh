@@ -4,7 +4,7 @@
 //
 //   fit_mean_kernel   tile-averaged ISF per (scale, lambda, tau) (the script's ISF_scale,
 //                     plot_averaged.py:246-252)
-//   fit_isf_kernel    one thread per curve: I(tau) = A (1 - exp(-F tau)) + B (fit_func,
+//   fit_isf_kernel    one warp per curve: I(tau) = A (1 - exp(-F tau)) + B (fit_func,
 //                     :57-58) by Levenberg-Marquardt in FP64, from the script's fixed starting
 //                     point p0 = (F, A, B) = (6, 0.03, 0.004) (:77) or from one read off the
 //                     curve (fit_start_from_data), with the covariance scaling of
@@ -20,6 +20,13 @@
 // retry with mu * 10; stop when a step changes the cost by less than 1e-15 of itself or the
 // parameters by less than 1e-13 of themselves, or after kFitMaxIter iterations. The model's
 // Jacobian is analytic. exp arguments are capped at 700, as the script's where= guard does.
+//
+// A warp per curve. A fit is a serial chain of evaluations, each a sum over the taus of terms with
+// an FP64 exponential: with one thread per curve (a few thousand threads on the GPU) the chain of
+// exponentials was all the time (7.1 ms for the 2,670 curves of 512^2, four scales, 64 taus, 30
+// lambdas; 148 SMs nearly idle). Here the lanes evaluate the terms of kFitBlock taus at once and ten
+// of them then add up one sum each in tau order, so every sum has the bits of the serial loop; the
+// 3 x 3 step is computed by all lanes alike.
 #pragma once
 
 #include <cstdint>
@@ -28,6 +35,9 @@
 namespace ddm {
 
 constexpr int kFitThreads = 128;
+constexpr int kFitBlock = 64;   // taus whose terms a warp holds at once
+constexpr int kFitSums = 10;    // cost, J^T J (6), J^T r (3)
+constexpr int kFitWarps = kFitThreads / 32;
 constexpr int kFitMaxIter = 400;
 constexpr int kFitParams = 6;  // F, A, B, sigma_F, sigma_A, sigma_B per curve
 
@@ -60,25 +70,39 @@ __global__ void fit_mean_kernel(FitArgs a) {
 
 __device__ __forceinline__ double fit_exp(double x) { return exp(x < 700.0 ? x : 700.0); }
 
-// Sum of squared residuals of (F, A, B) over the curve, and optionally J^T J and J^T r.
-__device__ double fit_eval(const double *y, const double *tau, int T, const double p[3], double H[6],
-                           double g[3], bool jac) {
-    double cost = 0.0;
-    if (jac) {
-        for (int i = 0; i < 6; i++) H[i] = 0.0;
-        for (int i = 0; i < 3; i++) g[i] = 0.0;
-    }
-    for (int i = 0; i < T; i++) {
-        const double e = fit_exp(-p[0] * tau[i]);
-        const double r = p[1] * (1.0 - e) + p[2] - y[i];
-        cost += r * r;
-        if (jac) {
-            const double j0 = p[1] * tau[i] * e, j1 = 1.0 - e, j2 = 1.0;
-            H[0] += j0 * j0, H[1] += j0 * j1, H[2] += j0 * j2;  // symmetric 3x3: 00 01 02 11 12 22
-            H[3] += j1 * j1, H[4] += j1 * j2, H[5] += j2 * j2;
-            g[0] += j0 * r, g[1] += j1 * r, g[2] += j2 * r;
+struct FitTerms {  // of one warp: residual and Jacobian of kFitBlock taus, and the finished sums
+    double r[kFitBlock], j0[kFitBlock], j1[kFitBlock];
+    double sum[kFitSums];
+};
+
+// Sum of squared residuals of (F, A, B) over the curve, J^T J (symmetric 3x3: 00 01 02 11 12 22) and
+// J^T r, by one warp: lane 0 adds up the cost, lanes 1..6 H, lanes 7..9 g, each in tau order.
+__device__ double fit_eval(const double *y, const double *tau, int T, const double p[3], FitTerms &w, double H[6],
+                           double g[3]) {
+    const int lane = threadIdx.x & 31;
+    // the factors of each lane's products: r, j0, j1 or j2 = 1
+    const double *left = lane == 0 || lane >= 7 ? w.r : lane <= 3 ? w.j0 : lane <= 5 ? w.j1 : nullptr;
+    const double *right = lane == 0 ? w.r : lane == 1 || lane == 7 ? w.j0 : lane == 2 || lane == 4 || lane == 8 ? w.j1 : nullptr;
+    double sum = 0.0;
+    for (int i0 = 0; i0 < T; i0 += kFitBlock) {
+        const int n = min(kFitBlock, T - i0);
+        for (int i = lane; i < n; i += 32) {
+            const double e = fit_exp(-p[0] * tau[i0 + i]);
+            w.r[i] = fma(p[1], 1.0 - e, p[2]) - y[i0 + i];
+            w.j0[i] = p[1] * tau[i0 + i] * e;
+            w.j1[i] = 1.0 - e;
         }
+        __syncwarp();
+        if (lane < kFitSums)
+            for (int i = 0; i < n; i++) sum = fma(left ? left[i] : 1.0, right ? right[i] : 1.0, sum);
+        __syncwarp();
     }
+    if (lane < kFitSums) w.sum[lane] = sum;
+    __syncwarp();
+    const double cost = w.sum[0];
+    for (int i = 0; i < 6; i++) H[i] = w.sum[1 + i];
+    for (int i = 0; i < 3; i++) g[i] = w.sum[7 + i];
+    __syncwarp();  // the sums are rewritten by the next evaluation
     return cost;
 }
 
@@ -115,11 +139,11 @@ __device__ void fit_start_from_data(const double *y, const double *tau, int T, d
     p[2] = b;
 }
 
-__device__ void fit_curve(const double *y, const double *tau, int T, int start, double out[kFitParams]) {
+__device__ void fit_curve(const double *y, const double *tau, int T, int start, FitTerms &w, double out[kFitParams]) {
     double p[3] = {6.0, 3e-2, 4e-3};  // plot_averaged.py:77
     if (start == 0) fit_start_from_data(y, tau, T, p);
     double H[6], g[3];
-    double cost = fit_eval(y, tau, T, p, H, g, true);
+    double cost = fit_eval(y, tau, T, p, w, H, g);
     double mu = 1e-3;
     for (int it = 0; it < kFitMaxIter; it++) {
         bool accepted = false, done = false;
@@ -133,7 +157,7 @@ __device__ void fit_curve(const double *y, const double *tau, int T, int start, 
             }
             const double pn[3] = {p[0] + d[0], p[1] + d[1], p[2] + d[2]};
             double Hn[6], gn[3];
-            const double cn = fit_eval(y, tau, T, pn, Hn, gn, true);
+            const double cn = fit_eval(y, tau, T, pn, w, Hn, gn);
             if (isfinite(cn) && cn <= cost) {
                 const bool small_step = fabs(d[0]) <= 1e-13 * fabs(p[0]) && fabs(d[1]) <= 1e-13 * fabs(p[1]) &&
                                         fabs(d[2]) <= 1e-13 * (fabs(p[2]) + 1e-300);
@@ -163,10 +187,11 @@ __device__ void fit_curve(const double *y, const double *tau, int T, int start, 
     }
 }
 
-__global__ void fit_isf_kernel(FitArgs a) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kFitThreads) fit_isf_kernel(FitArgs a) {
+    __shared__ FitTerms terms[kFitWarps];
+    const int c = blockIdx.x * kFitWarps + (threadIdx.x >> 5);
     const int total = a.tile_curves + a.S * a.Q;
-    if (c >= total) return;
+    if (c >= total) return;  // whole warps
     const double *y;
     double *out;
     if (c < a.tile_curves) {
@@ -181,8 +206,9 @@ __global__ void fit_isf_kernel(FitArgs a) {
         out = a.scale_fit + static_cast<long long>(sc) * kFitParams;
     }
     double r[kFitParams];
-    fit_curve(y, a.tau, a.T, a.start, r);
-    for (int i = 0; i < kFitParams; i++) out[i] = r[i];
+    fit_curve(y, a.tau, a.T, a.start, terms[threadIdx.x >> 5], r);
+    if ((threadIdx.x & 31) == 0)
+        for (int i = 0; i < kFitParams; i++) out[i] = r[i];
 }
 
 // One thread per (scale, tile) and per scale: D from the Q decay rates of its curves.
