@@ -23,6 +23,7 @@
 #include "../../include/ddm.h"
 #include "engine_internal.hpp"
 #include "errors.hpp"
+#include "host_copy.hpp"
 #include "lag.cuh"
 #include "lag_hist.cuh"
 #include "pinned_pool.hpp"
@@ -580,7 +581,7 @@ extern "C" int ddm_server_poll(ddm_server *s, int stream_id, ddm_chunk_result *r
         return fail(DDM_ERR_CUDA, std::string(device_status_text(*slot->status_h)) + "; results are incomplete");
     if (isf) {
         if (capacity < st.isf_size) return fail(DDM_ERR_INVALID_ARG, "ddm_server_poll: ISF buffer too small");
-        std::memcpy(isf, slot->isf_h, sizeof(double) * st.isf_size);
+        parallel_copy(isf, slot->isf_h, sizeof(double) * st.isf_size);
     }
     if (res) {
         res->chunk_index = slot->chunk_index;
