@@ -324,10 +324,23 @@ __device__ __forceinline__ void lag_hist_body(const HistTarget &tgt, const int *
                             for (int j = 0; j < J; j++)
                                 c[j & 3] = hist_diff_sq_acc(*reinterpret_cast<const float2 *>(w + j * kHistRowBytes), x[j], c[j & 3]);
                         } else {
+                            // by eights: a whole one (in both halves) needs no test per pair
 #pragma unroll
-                            for (int j = 0; j < J; j++)
-                                if (st.z & (1u << j))
-                                    c[j & 3] = hist_diff_sq_acc(*reinterpret_cast<const float2 *>(w + j * kHistRowBytes), x[j], c[j & 3]);
+                            for (int j0 = 0; j0 < J; j0 += 8) {
+                                constexpr unsigned kEight = 255;
+                                const unsigned all = j0 + 8 <= J ? kEight : kEight >> (j0 + 8 - J);
+                                const unsigned part = (static_cast<unsigned>(st.z) >> j0) & all;
+                                if (__all_sync(0xffffffffu, part == all)) {
+#pragma unroll
+                                    for (int j = j0; j < j0 + 8 && j < J; j++)
+                                        c[j & 3] = hist_diff_sq_acc(*reinterpret_cast<const float2 *>(w + j * kHistRowBytes), x[j], c[j & 3]);
+                                } else if (part) {
+#pragma unroll
+                                    for (int j = j0; j < j0 + 8 && j < J; j++)
+                                        if (part & (1u << (j - j0)))
+                                            c[j & 3] = hist_diff_sq_acc(*reinterpret_cast<const float2 *>(w + j * kHistRowBytes), x[j], c[j & 3]);
+                                }
+                            }
                         }
                         const float sum = ((c[0].x + c[0].y) + (c[1].x + c[1].y)) + ((c[2].x + c[2].y) + (c[3].x + c[3].y));
                         const float y = sum - a.y;

@@ -218,7 +218,7 @@ inline std::string build_hist_table(const HistInput &in, int EB, int CW, int buf
                     const int need = stages_of(top.row + (variants > 1 ? b : 0) * nreg + nreg +
                                                (u.kind == kHistRun ? kLagFuse - 1 : 0));
                     const bool active = h == 0 || l[s].both;
-                    const int mask = u.kind == kHistRun ? u.mask * kHistRowBytes : active || u.kind == kHistFull ? u.mask : 0;
+                    const int mask = u.kind == kHistRun ? u.mask * kHistRowBytes : u.mask;
                     steps.push_back(HistStep{u.row * kHistRowBytes, u.acc * kHistRowBytes, mask,
                                              u.kind | (active ? kHistActive : 0) | need << kHistNeedShift | below << kHistRelShift});
                 }

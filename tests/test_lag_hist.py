@@ -165,7 +165,9 @@ def check_pairs(c, t):
                 kind, row = info & 3, row + b * nreg
                 ready = rows_of(t, max((info >> 4) & 15, t["sub_stages"][b] if b and t["variants"] == 1 or not t["nx"]
                                        else 0))
-                assert (kind or mask) if info & 4 else (kind or not mask)
+                assert kind or mask
+                if not kind:
+                    assert {row + j for j in range(nreg) if (mask >> j) & 1} <= ready
                 if kind:  # every row read has landed
                     assert set(range(row, row + nreg + (LENGTH[kind] - 1))) <= ready
                 if kind == 1:
