@@ -59,10 +59,13 @@ namespace {
 
 constexpr int kTables = 64;  // lag tables in flight
 constexpr int kAsyncMax = 8;  // ddm_finalize_async result slots (ddm_set_async_depth)
+constexpr int kLagDone = 8;  // lag launches an FFT can wait for one by one
 constexpr int kSubmitEvents = 8;  // submit calls ddm_wait_frames_copied can look back over
 
-struct Launch {  // one lag-kernel launch: register frames, tau windows (ascending), position slots
-    int nreg = 0;
+// One lag-kernel launch: register frames, tau windows (ascending), position slots. nsub > 1: so many
+// sub-batches of nreg frames one after another (windows nreg positions further each).
+struct Launch {
+    int nreg = 0, nsub = 1;
     int reg[kMaxJ];
     std::vector<int> ent_acc, ent_w, pos;
 };
@@ -164,6 +167,13 @@ struct ddm_engine {
     int inject = DDM_FAULT_NONE;            // one-shot fault for the next lag launch (ddm_inject_fault)
     LagMaps maps;                           // 2-D tensor maps of the ring for the lag kernel
     HistShape hist;                         // CTA shape of the resident-history lag kernel (EB 0: not used)
+    // Launches of two full batches (hist_pair.EB > 0) while a submit call has frames for them: the
+    // second reads only the frames the first did not. lag_done[i] follows a launch that reads ring
+    // labels from lag_oldest[i] on; an FFT that overwrites older labels waits for it.
+    HistShape hist_pair;
+    cudaEvent_t lag_done[kLagDone] = {};
+    long long lag_oldest[kLagDone] = {};
+    long long lag_launches = 0;
     RingLayout lay;                         // where a ring slot's elements live
     AccLayout acc_lay;                      // and the accumulators
     bool defer_lag = false;                 // served: lag launches are collected, not issued
@@ -248,6 +258,8 @@ void free_all(ddm_engine *e) {
         if (e->async_ev[i]) cudaEventDestroy(e->async_ev[i]);
     for (int i = 0; i < kSubmitEvents; i++)
         if (e->submit_ev[i]) cudaEventDestroy(e->submit_ev[i]);
+    for (cudaEvent_t ev : e->lag_done)
+        if (ev) cudaEventDestroy(ev);
     pinned_release(e->tables_h);
     for (int i = 0; i < kTables; i++) {
         if (e->tab_ev[i]) cudaEventDestroy(e->tab_ev[i]);
@@ -529,13 +541,15 @@ unsigned balanced_grid(unsigned blocks, unsigned resident) {
 int launch_hist(ddm_engine *e, const Launch &L) {
     HistInput in;
     in.nreg = L.nreg;
-    in.reg.assign(L.reg, L.reg + L.nreg);
+    in.nsub = L.nsub;
+    in.reg.assign(L.reg, L.reg + L.nreg * L.nsub);
     in.ent_acc = L.ent_acc;
     in.ent_w = L.ent_w;
     in.pos = L.pos;
     HistTable table;
-    const int EB = e->hist.EB, CW = e->hist.CW;
-    std::string err = build_hist_table(in, e->hist, &table);
+    const HistShape &shape = L.nsub > 1 ? e->hist_pair : e->hist;
+    const int EB = shape.EB, CW = shape.CW;
+    std::string err = build_hist_table(in, shape, &table);
     if (!err.empty()) return fail(DDM_ERR_STATE, "internal: " + err);
     if (table.steps == 0 && e->inject == DDM_FAULT_NONE) return DDM_OK;  // no frame has a partner yet
     if (e->inject == DDM_FAULT_LAG_WAIT) {
@@ -669,10 +683,11 @@ inline int slot_of(const ddm_engine *e, long long label) {
     return label < 0 ? -1 : static_cast<int>(label % e->R);
 }
 
-// Unbiased: the new frames n0 .. n0+c-1 pair with the frames tau before each.
-int lag_causal(ddm_engine *e, long long n0, int c) {
+// Unbiased: the new frames n0 .. n0+c-1 pair with the frames tau before each (in `nsub` sub-batches).
+int lag_causal(ddm_engine *e, long long n0, int c, int nsub = 1) {
     Launch L;
-    L.nreg = c;
+    L.nreg = c / nsub;
+    L.nsub = nsub;
     for (int j = 0; j < c; j++) L.reg[j] = slot_of(e, n0 + j);
     for (int i = e->T - 1; i >= 0; i--) {  // descending tau = ascending window start
         L.ent_acc.push_back(i);
@@ -686,7 +701,28 @@ int lag_causal(ddm_engine *e, long long n0, int c) {
         long long f = n0 - e->tau_max + p;
         L.pos[p] = f >= 0 ? slot_of(e, f) : -1;
     }
-    return launch_lag(e, L);
+    int st = launch_lag(e, L);
+    if (!st && e->hist_pair.EB && !e->defer_lag) {
+        const int i = static_cast<int>(e->lag_launches++ % kLagDone);
+        // the launch this slot followed is the oldest of kLagDone: no FFT looks it up any more, so the
+        // next one waits for it whatever it overwrites
+        if (e->lag_launches > kLagDone) CUDA_TRY(cudaStreamWaitEvent(e->fft_stream, e->lag_done[i], 0));
+        e->lag_oldest[i] = n0 - e->tau_max;
+        CUDA_TRY(cudaEventRecord(e->lag_done[i], e->stream));
+    }
+    return st;
+}
+
+// Holds the FFT stream until no queued lag launch reads the ring slots that frames below `label`
+// overwrite.
+int wait_for_slots(ddm_engine *e, long long label) {
+    const long long lost = label - e->R;  // labels below this are overwritten
+    for (long long k = e->lag_launches - 1; k >= 0 && k >= e->lag_launches - kLagDone; k--)
+        if (e->lag_oldest[k % kLagDone] < lost) {  // launches run in order: the newest such one covers the rest
+            CUDA_TRY(cudaStreamWaitEvent(e->fft_stream, e->lag_done[k % kLagDone], 0));
+            break;
+        }
+    return DDM_OK;
 }
 
 // Unbiased: pair every frame still waiting for a lag launch (compat runs the reference's
@@ -1022,6 +1058,24 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
         e->hist = hist_pick_shape(steady);
         if (e->hist.EB)
             e->tab_stride = std::max(e->tab_stride, hist_table_capacity(e->T, e->tau_max + e->lag_batch, 1));
+        // Two batches per launch where the ring holds both and the batches do not depend on how the
+        // frames arrive (a batch smaller than the ingest piece is cut at every piece). 64 taus up to 500
+        // at 1024^2, four scales: 1.85 ms per 32 frames one by one, 1.40 in pairs. Small launches gain
+        // more from running beside the next piece's FFT, which must wait for the longer launch (200
+        // frames of 256^2, 20 taus: 233 us one by one, 253 in pairs).
+        constexpr double kPairMinWork = 16e6;  // elements x taus: about 150 us per launch
+        if (e->hist.EB && !compat && e->G == 0 && e->lag_batch >= e->jmax &&
+            e->R - e->tau_max >= 2 * e->lag_batch && static_cast<double>(e->E) * e->T >= kPairMinWork) {
+            steady.nsub = 2;
+            for (int p = 0; p < e->lag_batch; p++) steady.pos.push_back((e->tau_max + e->lag_batch + p) % e->R);
+            steady.reg.assign(steady.pos.begin() + first, steady.pos.end());
+            e->hist_pair = hist_pick_shape(steady);
+            if (e->hist_pair.EB)
+                e->tab_stride = std::max(e->tab_stride, hist_table_capacity(e->T, e->tau_max + 2 * e->lag_batch, 2));
+            for (int i = 0; e->hist_pair.EB && i < kLagDone; i++)
+                if (cudaEventCreateWithFlags(&e->lag_done[i], cudaEventDisableTiming) != cudaSuccess)
+                    return bail(fail(DDM_ERR_CUDA, "cudaEventCreate failed"));
+        }
     }
     if (e->hist.EB) {
         e->lay = RingLayout{(e->E + 15) / 16 * 16, e->R, 1};
@@ -1162,6 +1216,7 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
                              static_cast<int>(fft_tile_smem_bytes(128))) != cudaSuccess ||
         cudaFuncSetAttribute(fft_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
         set_lag_limits(e->hist) != cudaSuccess ||
+        (e->hist_pair.EB && set_lag_limits(e->hist_pair) != cudaSuccess) ||
         cudaFuncSetAttribute(dft_bf16_kernel<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft_smem_bytes(32)) != cudaSuccess ||
         cudaFuncSetAttribute(dft_bf16_kernel<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft_smem_bytes(64)) != cudaSuccess ||
         cudaFuncSetAttribute(dft_bf16_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft_smem_bytes(128)) != cudaSuccess)
@@ -1221,8 +1276,14 @@ extern "C" int ddm_submit_frames(ddm_engine *e, const void *frames, int count, i
             const long long to_edge = period - e->submitted % period;
             piece = static_cast<int>(std::min<long long>(piece, to_edge));
         }
+        const bool pairs = e->hist_pair.EB && !e->defer_lag;
+        if (pairs) {  // the ring holds the frames that wait for their batches and this piece
+            const long long room = e->R - e->tau_max - (e->submitted - e->lag_next);
+            piece = static_cast<int>(std::min<long long>(piece, room));
+        }
         const uint8_t *p = src + frame_bytes * done;
         int st;
+        if (pairs && (st = wait_for_slots(e, e->submitted + piece))) return st;
         // hold this piece's FFT until every lag issued before the previous piece's FFT is done
         if (e->pieces > 0) CUDA_TRY(cudaStreamWaitEvent(e->fft_stream, e->ev_guard[(e->pieces - 1) & 1], 0));
         CUDA_TRY(cudaEventRecord(e->ev_guard[e->pieces & 1], e->stream));
@@ -1271,11 +1332,16 @@ extern "C" int ddm_submit_frames(ddm_engine *e, const void *frames, int count, i
         if (compat) {
             if ((st = run_ready_iterations(e, false))) return st;
         } else {
-            while (e->submitted - e->lag_next >= e->lag_batch) {
+            const bool more = pairs && done + piece < count;  // frames of this call still to come
+            while (pairs && e->submitted - e->lag_next >= 2 * e->lag_batch) {
+                if ((st = lag_causal(e, e->lag_next, 2 * e->lag_batch, 2))) return st;
+                e->lag_next += 2 * e->lag_batch;
+            }
+            while (!more && e->submitted - e->lag_next >= e->lag_batch) {
                 if ((st = lag_causal(e, e->lag_next, e->lag_batch))) return st;
                 e->lag_next += e->lag_batch;
             }
-            if (e->lag_batch <= e->jmax && (st = flush_lag(e))) return st;  // no batching
+            if (!more && e->lag_batch <= e->jmax && (st = flush_lag(e))) return st;  // no batching
             if (e->G > 0 && e->submitted % (static_cast<long long>(e->G) * e->C) == 0) {
                 if ((st = flush_lag(e))) return st;
                 if ((st = snapshot(e, e->pair_count))) return st;
@@ -1412,18 +1478,19 @@ extern "C" int ddm_wait_isf(ddm_engine *e) {
 // Device -> host copy of a large result on the engine's stream, done when it returns. Into pageable
 // memory it goes in two page-locked pieces, one arriving while the other is copied on by several
 // threads (a plain copy of 84 MB into fresh memory took 18 ms, mostly the driver's one thread
-// touching new pages); page-locked destinations and small results are copied directly.
+// touching new pages; 1 MB took 200 us); page-locked destinations and small results are copied directly.
 static int copy_result(ddm_engine *e, void *dst, const void *src, size_t bytes) {
-    constexpr size_t kPiece = 4u << 20;
+    constexpr size_t kPiece = 4u << 20, kDirect = 128u << 10;
     cudaPointerAttributes at;
     const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
     char *piece[2] = {nullptr, nullptr};
-    if (pageable && bytes >= 2 * kPiece) {
+    const size_t pieces = (bytes + kPiece - 1) / kPiece;
+    if (pageable && bytes >= kDirect) {
         piece[0] = static_cast<char *>(pinned_alloc(kPiece));
-        piece[1] = static_cast<char *>(pinned_alloc(kPiece));
+        if (pieces > 1) piece[1] = static_cast<char *>(pinned_alloc(kPiece));
     }
-    if (!piece[0] || !piece[1]) {
+    if (!piece[0] || (pieces > 1 && !piece[1])) {
         pinned_release(piece[0]);
         pinned_release(piece[1]);
         cudaGetLastError();
@@ -1432,7 +1499,6 @@ static int copy_result(ddm_engine *e, void *dst, const void *src, size_t bytes) 
         return DDM_OK;
     }
     cudaError_t err = cudaSuccess;
-    const size_t pieces = (bytes + kPiece - 1) / kPiece;
     auto size_of = [&](size_t i) { return std::min(kPiece, bytes - i * kPiece); };
     auto fetch = [&](size_t i) {
         return cudaMemcpyAsync(piece[i & 1], static_cast<const char *>(src) + i * kPiece, size_of(i),

@@ -321,3 +321,41 @@ def test_barrier_protocol_replay(probe):
         t = parse(c, line)
         if t["npiece"]:
             replay(c, t, 4, rng)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("side,scales,taus,chunk,calls", [
+    (64, [64, 32], log_taus(1, 40, 12), 7, (1, 6, 33, 20)),          # odd pieces, first frames without partners
+    (256, [256, 16], log_taus(1, 260, 64), 32, (40, 300, 5)),        # 16-element blocks, two buffers
+    (512, [512, 256, 128, 64], log_taus(1, 90, 40), 30, (200, 64, 31)),  # two batches per launch
+    (512, [512, 256, 128], log_taus(1, 620, 64), 17, (680, 130)),    # two CTAs per SM, two batches
+])
+def test_sums_match_float64(side, scales, taus, chunk, calls):
+    """Every lag sum of every spectrum element against the same sum in float64 over the engine's own
+    spectra: the launches' FP32 sums of up to 32 pairs round at most 2 * 32 times each (a difference,
+    a square and a sum per component), the Kahan sums over launches twice; so 1e-5 of the sum of the
+    exact squares bounds the error with an order of magnitude to spare."""
+    import numpy as np
+    import torch
+    from cuda_multiddm_b200 import Engine, EngineConfig
+    rng = np.random.default_rng(side + chunk)
+    n = sum(calls)
+    frames = rng.integers(0, 256, (n, side, side), dtype=np.uint8)
+    with Engine(EngineConfig(frame_width=side, frame_height=side, scales=scales, taus=taus, lambdas=[4.0, 8.0],
+                             chunk_frames=chunk)) as eng:
+        spec, done = [], 0
+        for c in calls:
+            eng.submit(frames[done:done + c])
+            done += c
+        got = eng.accumulators()
+    x = torch.from_numpy(frames.astype(np.float64)).cuda()
+    F = torch.cat([torch.fft.rfft2(x.view(n, side // s, s, side // s, s).permute(0, 1, 3, 2, 4)).reshape(n, -1)
+                   for s in sorted(scales, reverse=True)], 1)
+    for i, tau in enumerate(taus):
+        want = torch.zeros(F.shape[1], dtype=torch.float64, device="cuda")
+        for t in range(tau, n):
+            want += torch.view_as_real(F[t] - F[t - tau]).square().sum(-1)
+        err = (torch.from_numpy(got[i]).cuda() - want).abs()
+        scale = want + (n - tau) * (1e-6 * F.abs().amax()) ** 2 + 1e-30  # spectra: 1e-6 of the largest value
+        spectra = 2 * torch.sqrt(want * max(n - tau, 0)) * 2e-6 * F.abs().amax()  # their effect on a sum
+        assert bool((err <= 1e-5 * scale + spectra).all()), (tau, float((err / scale).max()))
