@@ -347,7 +347,8 @@ __global__ void __launch_bounds__(kDftThreads, 1) dft_bf16_kernel(DftArgs a) {
                 }
             }
             __syncthreads();
-            const FramePtr frame(a.ring, a.lay, static_cast<int>((a.first_label + f) % a.lay.R));
+            const int slot = static_cast<int>((a.first_label + f) % a.lay.R);
+            const FramePtr<false> frame(a.ring + a.lay.base(slot), a.lay.stride(slot));
             const int ntl = tiles - b * TPB < TPB ? tiles - b * TPB : TPB;
             // sc.n = S * NX is even: every tile starts at an even element, and pairs of elements are
             // 16 aligned bytes of one element block

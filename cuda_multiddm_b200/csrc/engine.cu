@@ -5,7 +5,9 @@
 //   ring   float2 [R][E]   spectra of the last R frames; frame label f lives in slot f % R.
 //                          A frame is the concatenation over scales (descending) of
 //                          [tile][ky][kx], kx in [0, s/2]; E = sum_s tiles_s * s * (s/2+1).
-//   acc    float2 [T][E]   per (tau, element): FP32 running sum of |dF|^2 and its Kahan
+//                          Stored in slabs of 32 frames for the resident-history lag kernel,
+//                          else frame by frame (layout.cuh).
+//   acc    float2 [T][E]   (slabs: blocked alike) per (tau, element): FP32 running sum of |dF|^2 and its Kahan
 //                          compensation (true value = sum - comp), unnormalised.
 //   stage  uint8  [J][M][M*bpp]   ROI of host-submitted frames (one piece at a time).
 //   tables int    [kTables][tab_stride]  lag-kernel pair tables, a ring of slots.
@@ -388,6 +390,9 @@ int launch_fft(ddm_engine *e, const uint8_t *src, long long frame_stride, long l
         smem = std::max(smem, fft_smem_bytes(s));
     }
     rows.S = cols.S = nfft;
+    // The column pass writes neighbouring lines of a slab for neighbouring frames, so its CTAs take the
+    // frames of a few columns together (30 frames of 1024^2, four scales: 0.498 -> 0.462 ms).
+    cols.frames_first = e->lay.slabs && e->fft_mid && col_ctas <= 65535;
     // Frames go through both passes in groups of up to 256 MB of spectra (15 frames of the
     // 1024^2 x 4-scale shape): fewer, larger launches were measured faster than groups small
     // enough for the row pass's output to stay in L2 (frames/s at 34 / 64 / 100 / 256 MB:
@@ -422,9 +427,14 @@ int launch_fft(ddm_engine *e, const uint8_t *src, long long frame_stride, long l
             tr.e->tlaunch[0] += 1;
         }
         if (nfft > 0) {
-            fft_rows_kernel<<<dim3(row_ctas, nf), kFftThreads, smem, e->fft_stream>>>(rows);
+            const dim3 row_grid(row_ctas, nf), col_grid = cols.frames_first ? dim3(nf, col_ctas) : dim3(col_ctas, nf);
+            const bool ring_linear = !e->lay.slabs, mid_linear = ring_linear || e->fft_mid;
+            (mid_linear ? fft_rows_kernel<true> : fft_rows_kernel<false>)<<<row_grid, kFftThreads, smem, e->fft_stream>>>(
+                rows);
             CUDA_TRY(cudaGetLastError());
-            fft_cols_kernel<<<dim3(col_ctas, nf), kFftThreads, smem, e->fft_stream>>>(cols);
+            (ring_linear  ? fft_cols_kernel<true, true>
+             : mid_linear ? fft_cols_kernel<true, false>
+                          : fft_cols_kernel<false, false>)<<<col_grid, kFftThreads, smem, e->fft_stream>>>(cols);
             CUDA_TRY(cudaGetLastError());
             e->launches += 2;
             tr.e->tlaunch[0] += 2;
@@ -1207,14 +1217,17 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
     }
 
     // Kernel shared-memory limits (the FFT passes use up to 128 KB)
-    if (cudaFuncSetAttribute(fft_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
+    if (cudaFuncSetAttribute(fft_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(fft_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
         cudaFuncSetAttribute(fft_tile_kernel<5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(fft_tile_smem_bytes(32))) != cudaSuccess ||
         cudaFuncSetAttribute(fft_tile_kernel<6>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(fft_tile_smem_bytes(64))) != cudaSuccess ||
         cudaFuncSetAttribute(fft_tile_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(fft_tile_smem_bytes(128))) != cudaSuccess ||
-        cudaFuncSetAttribute(fft_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(fft_cols_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(fft_cols_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(fft_cols_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
         set_lag_limits(e->hist) != cudaSuccess ||
         (e->hist_pair.EB && set_lag_limits(e->hist_pair) != cudaSuccess) ||
         cudaFuncSetAttribute(dft_bf16_kernel<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft_smem_bytes(32)) != cudaSuccess ||

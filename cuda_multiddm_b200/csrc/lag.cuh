@@ -1,4 +1,5 @@
-// Lag kernel: accumulates |F(x) - F(y)|^2 for a block of J "register" frames x against
+// Ring lag kernel (engines whose history does not fit the resident-history kernel of lag_hist.cuh, and
+// the static entry point): accumulates |F(x) - F(y)|^2 for a block of J "register" frames x against
 // the partner frame y of every tau, per spectrum element (replaces processFFT,
 // src/DDM_kernel.cuh:85-101, which the reference launches once per (scale, tau, frame)).
 //

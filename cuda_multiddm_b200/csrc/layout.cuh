@@ -35,19 +35,19 @@ struct RingLayout {
     __host__ __device__ int stride(int slot) const { return slabs ? slab_height(slot) * 16 : 16; }
 };
 
-// One frame's elements: p[e] of the frame is at[e] below.
+// One frame's elements: element e is *at(e). LINEAR: one after another (a natural slot, or a buffer of
+// frames), else blocks of 16 a stride apart.
+template <bool LINEAR>
 struct FramePtr {
     float2 *p;
     int stride;
-    __device__ __forceinline__ FramePtr(float2 *ring, const RingLayout &l, int slot)
-        : p(ring + l.base(slot)), stride(l.stride(slot)) {}
     __device__ __forceinline__ FramePtr(float2 *first, int block_stride) : p(first), stride(block_stride) {}
     __device__ __forceinline__ float2 *at(int e) const {
-        return p + static_cast<long long>(e >> 4) * stride + (e & 15);
+        return LINEAR ? p + e : p + static_cast<long long>(e >> 4) * stride + (e & 15);
     }
-    // element e + d, given at = at(e), for a d known at compile time: whole blocks are a fixed distance
+    // element e + d, given at_e = at(e), for a d known at compile time: whole blocks are a fixed distance
     __device__ __forceinline__ float2 *step(float2 *at_e, int e, int d) const {
-        return d % 16 == 0 ? at_e + static_cast<long long>(d / 16) * stride : at(e + d);
+        return LINEAR ? at_e + d : d % 16 == 0 ? at_e + static_cast<long long>(d / 16) * stride : at(e + d);
     }
 };
 

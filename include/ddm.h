@@ -88,8 +88,9 @@ typedef struct {
                                       every scale (the reference uses cuFFT in FP32 for all,
                                       src/DDM.cu:648-677). Other scales always use the FP32 FFT. */
     int lag_geometry;              /* lag-kernel geometry for launches of up to 32 frames:
-                                      0 = one thread per spectrum element, four consumer warps
-                                      and three CTAs per SM; 1 = two threads per element (half
+                                      0 = the lag history of 16 or 32 elements resident in shared
+                                      memory (where it does not fit, or for fewer than 8 taus: one
+                                      thread per spectrum element and a ring of partner frames); 1 = two threads per element (half
                                       the frames each), eight consumer warps and two CTAs per SM.
                                       The same pairs, their FP32 sums formed in another order
                                       (both within 1e-5 of the FP64 oracle). With
