@@ -284,7 +284,7 @@ void free_all(ddm_engine *e) {
     for (cudaEvent_t ev : e->ev_guard)
         if (ev) cudaEventDestroy(ev);
     stream_release(e->device, e->fft_stream);
-    if (e->own_stream) stream_release(e->device, e->stream);
+    if (e->own_stream) stream_release(e->device, e->stream, true);
 }
 
 // Brackets a group of launches with events when timing is on (group 0 FFT, 1 lag, 2 azimuth).
@@ -1038,7 +1038,9 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
     if (cfg->stream) {
         e->stream = static_cast<cudaStream_t>(cfg->stream);
     } else {
-        if (!(e->stream = stream_acquire(e->device))) return bail(fail(DDM_ERR_CUDA, "cudaStreamCreate failed"));
+        // The greatest priority: the persistent lag CTAs find their places before the next piece's FFT
+        // takes them for thousands of short blocks (a CTA that starts late holds up the whole launch).
+        if (!(e->stream = stream_acquire(e->device, true))) return bail(fail(DDM_ERR_CUDA, "cudaStreamCreate failed"));
         e->own_stream = true;
     }
     // private streams from the process-wide pool (creating streams while the device is busy

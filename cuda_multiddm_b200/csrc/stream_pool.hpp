@@ -20,11 +20,12 @@ class StreamPool {
         static StreamPool pool;  // lives until exit; the driver releases the streams then
         return pool;
     }
-    // A non-blocking stream of `device` (the calling thread's current device), or nullptr.
-    cudaStream_t acquire(int device) {
+    // A non-blocking stream of `device` (the calling thread's current device), or nullptr; `first`: of
+    // the greatest priority, whose blocks are placed before those of the other streams.
+    cudaStream_t acquire(int device, bool first = false) {
         {
             std::lock_guard<std::mutex> g(lock_);
-            auto &fl = free_[device];
+            auto &fl = first ? first_[device] : free_[device];
             if (!fl.empty()) {
                 cudaStream_t s = fl.back();
                 fl.pop_back();
@@ -32,13 +33,15 @@ class StreamPool {
             }
         }
         cudaStream_t s = nullptr;
-        if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
+        int least = 0, greatest = 0;
+        if (first && cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess) return nullptr;
+        if (cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, greatest) != cudaSuccess) return nullptr;
         return s;
     }
-    void release(int device, cudaStream_t s) {
+    void release(int device, cudaStream_t s, bool first = false) {
         if (!s) return;
         std::lock_guard<std::mutex> g(lock_);
-        free_[device].push_back(s);
+        (first ? first_ : free_)[device].push_back(s);
     }
     // Makes at least n streams of `device` (the current device) idle in the pool.
     void reserve(int device, int n) {
@@ -58,10 +61,10 @@ class StreamPool {
 
   private:
     std::mutex lock_;
-    std::map<int, std::vector<cudaStream_t>> free_;
+    std::map<int, std::vector<cudaStream_t>> free_, first_;
 };
 
-inline cudaStream_t stream_acquire(int device) { return StreamPool::get().acquire(device); }
-inline void stream_release(int device, cudaStream_t s) { StreamPool::get().release(device, s); }
+inline cudaStream_t stream_acquire(int device, bool first = false) { return StreamPool::get().acquire(device, first); }
+inline void stream_release(int device, cudaStream_t s, bool first = false) { StreamPool::get().release(device, s, first); }
 
 }  // namespace ddm
