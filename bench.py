@@ -152,7 +152,7 @@ def profiled_traffic(w: dict, frames: float):
     figure in the committed capture of the headline workload (None for other workloads)."""
     if w is not WORKLOADS["c2"]:
         return None, None
-    p = ROOT / "profiles" / "lag_kernel_c2.txt"
+    p = ROOT / "profiles" / "lag_hist_c2.txt"
     if not p.exists():
         return None, None
     src, per_frame = None, None
@@ -428,7 +428,7 @@ def run_ours(args, w: dict) -> None:
                                 "frame_spectra_mb": frames_elements(w) * 8 / 1e6},
                 "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": CHUNK * side * side * bpp,
                         "d2h_bytes_per_step": isf_bufs[0].nbytes},
-                "roofline": {"bound": "hbm", "kernel": "lag_pipe_kernel", "achieved": achieved, "peak": hbm_peak,
+                "roofline": {"bound": "hbm", "kernel": "lag_hist_kernel", "achieved": achieved, "peak": hbm_peak,
                              "unit": "GB/s", "frac": achieved / hbm_peak, "peak_kind": peak_kind,
                              "traffic": traffic_total / per_launch if traffic_total else None,
                              "traffic_source": traffic_src,
