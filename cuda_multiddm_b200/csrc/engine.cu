@@ -392,7 +392,10 @@ int launch_fft(ddm_engine *e, const uint8_t *src, long long frame_stride, long l
     rows.S = cols.S = nfft;
     // The column pass writes neighbouring lines of a slab for neighbouring frames, so its CTAs take the
     // frames of a few columns together (30 frames of 1024^2, four scales: 0.498 -> 0.462 ms).
-    cols.frames_first = e->lay.slabs && e->fft_mid && col_ctas <= 65535;
+    // Groups that stay in L2 gain nothing from it.
+    constexpr double kFramesFirstMin = 32.0 * (1 << 20);
+    cols.frames_first = e->lay.slabs && e->fft_mid && col_ctas <= 65535 &&
+                        static_cast<double>(sizeof(float2)) * e->E * nframes >= kFramesFirstMin;
     // Frames go through both passes in groups of up to 256 MB of spectra (15 frames of the
     // 1024^2 x 4-scale shape): fewer, larger launches were measured faster than groups small
     // enough for the row pass's output to stay in L2 (frames/s at 34 / 64 / 100 / 256 MB:
@@ -1496,19 +1499,24 @@ extern "C" int ddm_wait_isf(ddm_engine *e) {
 // touching new pages; 1 MB took 200 us); page-locked destinations and small results are copied directly.
 static int copy_result(ddm_engine *e, void *dst, const void *src, size_t bytes) {
     constexpr size_t kPiece = 4u << 20, kDirect = 128u << 10;
-    cudaPointerAttributes at;
-    const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
-    cudaGetLastError();
+    bool pageable = false;
+    if (bytes >= kDirect) {
+        cudaPointerAttributes at;
+        pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+        cudaGetLastError();
+    }
     char *piece[2] = {nullptr, nullptr};
     const size_t pieces = (bytes + kPiece - 1) / kPiece;
-    if (pageable && bytes >= kDirect) {
+    if (pageable) {
         piece[0] = static_cast<char *>(pinned_alloc(kPiece));
         if (pieces > 1) piece[1] = static_cast<char *>(pinned_alloc(kPiece));
     }
     if (!piece[0] || (pieces > 1 && !piece[1])) {
-        pinned_release(piece[0]);
-        pinned_release(piece[1]);
-        cudaGetLastError();
+        if (pageable) {
+            pinned_release(piece[0]);
+            pinned_release(piece[1]);
+            cudaGetLastError();
+        }
         CUDA_TRY(cudaStreamSynchronize(e->stream));
         CUDA_TRY(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost));
         return DDM_OK;

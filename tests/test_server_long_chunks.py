@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("taus", [media.log_taus(1, 40, 12), [1, 2, 3, 5, 8]])
 def test_long_chunks_equal_the_engine_alone(taus):
-    C, chunks, side = 80, 3, 128
+    C, chunks, side = 64, 3, 128
     cfg = dict(frame_width=side, frame_height=side, scales=[128, 32], taus=taus, lambdas=[4.0, 8.0, 16.0],
                chunk_frames=C, lag_batch_frames=32)
     video = media.synth_video(9, side, side, C * chunks, 80, step_var=1.0)
