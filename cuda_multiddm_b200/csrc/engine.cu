@@ -705,9 +705,6 @@ int lag_causal(ddm_engine *e, long long n0, int c, int nsub = 1) {
     for (int i = e->T - 1; i >= 0; i--) {  // descending tau = ascending window start
         L.ent_acc.push_back(i);
         L.ent_w.push_back(e->tau_max - e->taus[i]);
-        long long first = n0 - e->taus[i];  // partner of j = 0
-        long long valid = std::max<long long>(0, std::min<long long>(c, first + c));
-        e->pair_count[i] += static_cast<double>(valid);
     }
     L.pos.resize(c + e->tau_max);
     for (int p = 0; p < c + e->tau_max; p++) {
@@ -715,7 +712,12 @@ int lag_causal(ddm_engine *e, long long n0, int c, int nsub = 1) {
         L.pos[p] = f >= 0 ? slot_of(e, f) : -1;
     }
     int st = launch_lag(e, L);
-    if (!st && e->hist_pair.EB && !e->defer_lag) {
+    if (st) return st;
+    for (int i = 0; i < e->T; i++) {  // the pairs count once they are queued
+        const long long first = n0 - e->taus[i];  // partner of j = 0
+        e->pair_count[i] += static_cast<double>(std::max<long long>(0, std::min<long long>(c, first + c)));
+    }
+    if (e->hist_pair.EB && !e->defer_lag) {
         const int i = static_cast<int>(e->lag_launches++ % kLagDone);
         // the launch this slot followed is the oldest of kLagDone: no FFT looks it up any more, so the
         // next one waits for it whatever it overwrites
@@ -723,7 +725,7 @@ int lag_causal(ddm_engine *e, long long n0, int c, int nsub = 1) {
         e->lag_oldest[i] = n0 - e->tau_max;
         CUDA_TRY(cudaEventRecord(e->lag_done[i], e->stream));
     }
-    return st;
+    return DDM_OK;
 }
 
 // Holds the FFT stream until no queued lag launch reads the ring slots that frames below `label`
@@ -1061,16 +1063,7 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
     // Launches of up to 32 frames of geometry 0 run on the resident-history kernel where their
     // frames fit its shared memory, on a ring in slabs; the ring kernel keeps the others.
     if (e->lag_geom == 0 && e->lag_batch <= kHistMaxJ) {
-        HistInput steady;
-        steady.nreg = e->lag_batch;
-        for (int p = 0; p < e->tau_max + e->lag_batch; p++) steady.pos.push_back(p % e->R);
-        for (int i = 0; i < e->T; i++) {
-            steady.ent_acc.push_back(i);
-            steady.ent_w.push_back(compat ? e->taus[i] : e->tau_max - e->taus[e->T - 1 - i]);
-        }
-        const int first = compat ? 0 : e->tau_max;
-        steady.reg.assign(steady.pos.begin() + first, steady.pos.begin() + first + e->lag_batch);
-        e->hist = hist_pick_shape(steady);
+        e->hist = hist_pick_shape(hist_steady(e->taus, e->lag_batch, 1, e->R, compat), compat);
         if (e->hist.EB)
             e->tab_stride = std::max(e->tab_stride, hist_table_capacity(e->T, e->tau_max + e->lag_batch, 1));
         // Two batches per launch where the ring holds both and the batches do not depend on how the
@@ -1081,10 +1074,7 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
         constexpr double kPairMinWork = 16e6;  // elements x taus: about 150 us per launch
         if (e->hist.EB && !compat && e->G == 0 && e->lag_batch >= e->jmax &&
             e->R - e->tau_max >= 2 * e->lag_batch && static_cast<double>(e->E) * e->T >= kPairMinWork) {
-            steady.nsub = 2;
-            for (int p = 0; p < e->lag_batch; p++) steady.pos.push_back((e->tau_max + e->lag_batch + p) % e->R);
-            steady.reg.assign(steady.pos.begin() + first, steady.pos.end());
-            e->hist_pair = hist_pick_shape(steady);
+            e->hist_pair = hist_pick_shape(hist_steady(e->taus, e->lag_batch, 2, e->R, compat), compat);
             if (e->hist_pair.EB)
                 e->tab_stride = std::max(e->tab_stride, hist_table_capacity(e->T, e->tau_max + 2 * e->lag_batch, 2));
             for (int i = 0; e->hist_pair.EB && i < kLagDone; i++)

@@ -92,7 +92,7 @@ inline std::string build_hist_table(const HistInput &in, int EB, int CW, int buf
     }
     row_of[npos] = static_cast<int>(slots.size());
     const int reg_row = reg_pos >= 0 ? row_of[reg_pos] : 0;
-    const int nrows = static_cast<int>(slots.size());
+    const int nrows = out->rows = static_cast<int>(slots.size());
     // the last row each sub-batch reads
     int last_row[kHistMaxSub] = {0};
     for (int b = 0; b < nsub; b++) {
@@ -260,15 +260,15 @@ inline std::string build_hist_table(const HistInput &in, int EB, int CW, int buf
         }
     std::copy(lptr.begin(), lptr.end(), p);
     if (!steps.empty()) std::memcpy(t + steps_at, steps.data(), sizeof(HistStep) * steps.size());
-    out->rows = nrows;
     out->steps = static_cast<int>(steps.size());
     return std::string();
 }
 
-// Upper bound of a table's ints for ntau entries over `rows` resident rows (as many pieces at
-// worst) and nsub sub-batches.
-inline int hist_table_capacity(int ntau, int rows, int nsub) {
-    return kHtHeader + 2 * (rows + kHistMaxJ) + nsub * 12 + 1 + 3 + 4 * nsub * (ntau + 3);
+// Upper bound of a table's ints for ntau entries over resident rows in `pieces` pieces (as many as
+// rows at worst) and nsub sub-batches: every entry a unit of its own in every sub-batch, which is
+// what launches without fused runs take.
+inline int hist_table_capacity(int ntau, int pieces, int nsub) {
+    return kHtHeader + 2 * (pieces + kHistMaxJ) + nsub * 12 + 1 + 3 + 4 * nsub * (ntau + 3);
 }
 
 // How an engine's launches run: elements per block, consumer warps per CTA, row buffers, and
@@ -289,6 +289,44 @@ inline std::string build_hist_table(const HistInput &in, const HistShape &shape,
     return err;
 }
 
+// A full launch of an engine once every partner is there: its windows, in ring slots 0, 1, ... Compat:
+// the windows start at the register frames and reach forward, else they reach back.
+inline HistInput hist_steady(const std::vector<int> &taus, int batch, int nsub, int R, bool compat) {
+    HistInput in;
+    const int T = static_cast<int>(taus.size()), tau_max = taus.back();
+    in.nreg = batch;
+    in.nsub = nsub;
+    for (int p = 0; p < tau_max + nsub * batch; p++) in.pos.push_back(p % R);
+    for (int i = 0; i < T; i++) {
+        in.ent_acc.push_back(i);
+        in.ent_w.push_back(compat ? taus[i] : tau_max - taus[T - 1 - i]);
+    }
+    const int first = compat ? 0 : tau_max;
+    in.reg.assign(in.pos.begin() + first, in.pos.begin() + first + nsub * batch);
+    return in;
+}
+
+// Whether every launch with no more frames than `steady` fits a CTA of the shape, in one of the forms
+// build_hist_table falls back to: no launch has other rows than the steady one, but its table may be
+// several times as large (no fused runs without an instance for its frame count or with a partner
+// missing; a list per sub-batch). Its pieces start at a window that does not touch the one before it,
+// at the register frames, at the first frame there is, or at a slab's or the ring's first slot; with
+// `scattered` positions (compat schedules) anywhere.
+inline bool hist_always_fits(const HistInput &steady, const HistShape &shape, bool scattered) {
+    const int ntau = static_cast<int>(steady.ent_acc.size());
+    int starts = static_cast<int>(steady.pos.size()) / kSlab + 6;
+    for (int i = 1; i < ntau; i++) starts += steady.ent_w[i] > steady.ent_w[i - 1] + 1;
+    for (const bool x_buffers : {false, true}) {
+        HistTable t;
+        build_hist_table(steady, shape.EB, shape.CW, 1, x_buffers, &t);  // for its rows, whether it fits or not
+        if (t.rows == 0) continue;
+        const int ints = hist_table_capacity(ntau, scattered ? t.rows : std::min(t.rows, starts), steady.nsub);
+        if (hist_table_offset(shape.EB, 1, t.rows, x_buffers) + sizeof(int) * ints <= static_cast<size_t>(kHistSmemMax))
+            return true;
+    }
+    return false;
+}
+
 // The shape for launches like `steady` (every partner there): as many CTAs per SM as the rows
 // leave room for, with the widest block (a thread of a wider block walks more entries per load of
 // its register frames), and in their shared memory whole blocks in two or more row buffers, else
@@ -298,7 +336,9 @@ inline std::string build_hist_table(const HistInput &in, const HistShape &shape,
 // register-frame buffers. The ring kernel keeps short tau lists, whose blocks are too little work for
 // their barriers (5 taus up to 20: 130 us against 142), and those that one CTA per SM would run
 // without many taus (20 taus up to 1000: 393 us against 439; 64: 727 against 648).
-inline HistShape hist_pick_shape(const HistInput &steady) {
+// A shape is taken only if no launch of the engine can outgrow it (hist_always_fits): the ring's
+// layout follows the kernel, so there is no other one to go to later.
+inline HistShape hist_pick_shape(const HistInput &steady, bool scattered) {
     constexpr int kMinTaus = 8, kMinTausOneCta = 48;
     constexpr struct {
         int EB, CW, taus;
@@ -316,9 +356,10 @@ inline HistShape hist_pick_shape(const HistInput &steady) {
             return build_hist_table(steady, s.EB, s.CW, buffers, x_buffers, &t).empty() &&
                    t.smem <= static_cast<size_t>(hist_smem_limit(s.CW));
         };
-        for (int buffers = kHistMaxBuffers; buffers >= 2; buffers--)
-            if (fits(buffers, false)) return s;
-        if (fits(1, true) || (size.bare && fits(1, false))) return s;
+        bool found = false;
+        for (int buffers = kHistMaxBuffers; buffers >= 2 && !found; buffers--) found = fits(buffers, false);
+        found = found || fits(1, true) || (size.bare && fits(1, false));
+        if (found && hist_always_fits(steady, s, scattered)) return s;
     }
     return HistShape();
 }
