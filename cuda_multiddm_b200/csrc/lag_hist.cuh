@@ -39,7 +39,8 @@
 //
 // Sub-batches whose lists differ (the first frames of a stream, where partners are missing) are
 // separated by a barrier of the consumer warps, since another thread may then own an entry's
-// accumulator. Every wait is bounded as in lag.cuh and reports through *status.
+// accumulator. Every wait is bounded as in lag.cuh, with one outcome for the whole warp, and reports
+// through *status.
 #pragma once
 
 #include "lag.cuh"
@@ -115,6 +116,19 @@ __host__ __device__ constexpr size_t hist_table_offset(int EB, int buffers, int 
 __device__ __forceinline__ float2 hist_diff_sq_acc(float2 y, float2 x, float2 acc) {
     const float2 d = __ffma2_rn(x, make_float2(-1.f, -1.f), y);
     return __ffma2_rn(d, d, acc);
+}
+
+// mbar_wait_bounded by a whole warp, with one outcome: lanes that gave up alone would leave the others
+// in the warp's next vote or __syncwarp. Every lane observes the phase itself (it reads what landed).
+__device__ __forceinline__ bool hist_warp_wait(uint64_t *bar, uint32_t parity, long long limit) {
+    bool done = mbar_try_wait(bar, parity);
+    if (__all_sync(0xffffffffu, done)) return true;
+    const long long t0 = clock64();
+    for (;;) {
+        if (!done) done = mbar_try_wait(bar, parity);
+        if (__all_sync(0xffffffffu, done)) return true;
+        if (__any_sync(0xffffffffu, clock64() - t0 > limit)) return false;
+    }
 }
 
 template <int J, int EB, int CW>
@@ -194,8 +208,8 @@ __device__ __forceinline__ void lag_hist_body(const HistTarget &tgt, const int *
         bool ok = true;
         auto issue_x = [&](int n) {
             if (nx == 0 || n >= nblocks) return;
-            if (n > 1 && !mbar_wait_bounded(&xempty[n & 1], ((n >> 1) - 1) & 1, wait_cycles)) ok = false;
-            if (!__all_sync(0xffffffffu, ok)) return;
+            if (n > 1 && !hist_warp_wait(&xempty[n & 1], ((n >> 1) - 1) & 1, wait_cycles)) ok = false;
+            if (!ok) return;
             const int b16 = (block_begin + n * block_step) * kRegions;
             const int regions = nb16 - b16 < kRegions ? nb16 - b16 : kRegions;
             if (lane == 0) mbar_expect_tx(&xfull[n & 1], tab[kHtXBytes] * regions);
@@ -204,7 +218,7 @@ __device__ __forceinline__ void lag_hist_body(const HistTarget &tgt, const int *
         };
         int begun = -1, buf = 0, use = 0;  // of block n: its row buffer, and how often that has been filled before
         issue_x(0);
-        for (int n = 0; ok && n < nblocks && !*abort_flag; n++) {
+        for (int n = 0; ok && n < nblocks && !__any_sync(0xffffffffu, *abort_flag); n++) {
             const int b16 = (block_begin + n * block_step) * kRegions;
             const int regions = nb16 - b16 < kRegions ? nb16 - b16 : kRegions;
             if (lane < regions)  // the block's accumulators into L2, ahead of their use
@@ -215,8 +229,7 @@ __device__ __forceinline__ void lag_hist_body(const HistTarget &tgt, const int *
             issue_x(n + 1);
             unsigned char *dst = smem + buf * buffer_bytes;
             for (int st = 0; st < nstages && ok; st++) {
-                if (use > 0 && !mbar_wait_bounded(&empty[buf * kHistStages + st], (use - 1) & 1, wait_cycles)) ok = false;
-                ok = __all_sync(0xffffffffu, ok);
+                if (use > 0 && !hist_warp_wait(&empty[buf * kHistStages + st], (use - 1) & 1, wait_cycles)) ok = false;
                 if (!ok) break;
                 uint64_t *bar = &full[buf * kHistStages + st];
                 if (lane == 0) mbar_expect_tx(bar, tab[kHtBytes + st] * regions);
@@ -241,10 +254,17 @@ __device__ __forceinline__ void lag_hist_body(const HistTarget &tgt, const int *
         const int m = lane & 15;  // element within the 16-element block
         const int variants = tab[kHtVariants];
         unsigned char *acc_base = reinterpret_cast<unsigned char *>(tgt.acc + m);
-        bool ok = true;
+        // A lane whose wait runs out goes on with its warp to the end of the block: one that left alone would
+        // be missing from the warp's next vote or __syncwarp. Lane 0 makes no arrivals after such a wait (a
+        // release must not run ahead of its copy), so the producer's waits run out too, and at most a block's
+        // waits (one per stage, two of the register frames and the sub-batches) pass their limits.
+        bool late = false, arrives = lane == 0;
+        auto wait_for = [&](uint64_t *bar, uint32_t phase) {
+            if (!mbar_wait_bounded(bar, phase, wait_cycles)) late = true, arrives = false;
+        };
         int buf = 0;
         uint32_t parity = 0;  // of the row buffer's barriers
-        for (int n = 0, block = block_begin; ok && block < block_end; block += block_step, n++) {
+        for (int n = 0, block = block_begin; block < block_end; block += block_step, n++) {
             const int b16 = block * kRegions + region;
             const bool valid = b16 < nb16;
             unsigned char *acc_k = acc_base + static_cast<long long>(b16) * tgt.T * kHistRowBytes;
@@ -252,21 +272,19 @@ __device__ __forceinline__ void lag_hist_body(const HistTarget &tgt, const int *
             uint64_t *stage = &full[buf * kHistStages];
             int have = 0, released = 0;
             auto wait_stages = [&](int need) {
-                for (; ok && have < need; have++)
-                    if (!mbar_wait_bounded(&stage[have], parity, wait_cycles)) ok = false;
+                for (; have < need; have++) wait_for(&stage[have], parity);
             };
             auto release = [&](int rel) {
                 if (rel > released) {
                     __syncwarp();
-                    if (lane == 0)
+                    if (arrives)
                         for (int st = released; st < rel; st++) mbar_arrive(&empty[buf * kHistStages + st]);
                     released = rel;
                 }
             };
-            if (nx > 0) ok = mbar_wait_bounded(&xfull[n & 1], (n >> 1) & 1, wait_cycles);
-            for (int b = 0; ok && b < nsub; b++) {
+            if (nx > 0) wait_for(&xfull[n & 1], (n >> 1) & 1);
+            for (int b = 0; b < nsub; b++) {
                 if (b > 0 || nx == 0) wait_stages(tab[kHtSubStages + b]);
-                if (!ok) break;
                 const unsigned char *sub_rows = rows + b * nreg * kHistRowBytes;
                 float2 x[J];  // the sub-batch's register frames
                 {
@@ -282,16 +300,15 @@ __device__ __forceinline__ void lag_hist_body(const HistTarget &tgt, const int *
                     }
                     if (b == 0 && nx > 0) {
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&xempty[n & 1]);
+                        if (arrives) mbar_arrive(&xempty[n & 1]);
                     }
                 }
                 const int *lp = lptr + (variants > 1 ? b * CW : 0) + warp;
                 const int s1 = lp[1];
                 const bool last = b == nsub - 1;
-                                for (int s = lp[0]; s < s1; s++) {
+                for (int s = lp[0]; s < s1; s++) {
                     const int4 st = *reinterpret_cast<const int4 *>(steps + s * kHalves + half);
                     wait_stages((st.w >> kHistNeedShift) & kHistNeedMask);
-                    if (!ok) break;
                     if (last) release(st.w >> kHistRelShift);
                     const unsigned char *w = sub_rows + st.x;
                     unsigned char *ap = acc_k + st.y;
@@ -355,14 +372,14 @@ __device__ __forceinline__ void lag_hist_body(const HistTarget &tgt, const int *
                         if (mine) __stcg(reinterpret_cast<float2 *>(ap), make_float2(t, (t - a.x) - y));
                     }
                 }
-                if (ok && variants > 1 && !last) {
+                if (variants > 1 && !last) {
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(sub_done);
-                    ok = mbar_wait_bounded(sub_done, (n * (nsub - 1) + b) & 1, wait_cycles);
+                    if (arrives) mbar_arrive(sub_done);
+                    wait_for(sub_done, (n * (nsub - 1) + b) & 1);
                 }
             }
             wait_stages(tab[kHtSubStages + nsub - 1]);
-            if (!ok) {
+            if (__any_sync(0xffffffffu, late)) {
                 *abort_flag = 1;
                 break;
             }
