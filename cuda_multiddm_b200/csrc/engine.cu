@@ -1404,6 +1404,8 @@ std::vector<DeferredLag> engine_take_deferred(ddm_engine *e) {
     return out;
 }
 
+int engine_piece_frames(const ddm_engine *e) { return e->jmax; }
+
 LagTarget engine_lag_target(const ddm_engine *e) { return LagTarget{e->ring, e->acc, e->E, e->status_d, &e->maps}; }
 
 HistTarget engine_hist_target(const ddm_engine *e) {

@@ -36,6 +36,7 @@ struct LagTarget {  // what a lag launch of this engine reads and writes
 // for the caller to issue, on the engine's stream, after the work queued before them.
 void engine_defer_lag(ddm_engine *e, bool on);
 std::vector<DeferredLag> engine_take_deferred(ddm_engine *e);
+int engine_piece_frames(const ddm_engine *e);  // frames per FFT piece at most
 LagTarget engine_lag_target(const ddm_engine *e);
 HistTarget engine_hist_target(const ddm_engine *e);
 // Validation and sizing of ddm_open only: the device bytes checked against the HBM budget.

@@ -1,8 +1,8 @@
 // Serving many DDM streams on one GPU: admission by HBM footprint, per-stream device state
 // (FFT ring, accumulators) kept resident, and continuous batching: every step takes the
 // next pending chunk of every stream that has one, runs each stream's FFT, then ONE lag
-// launch (per register-frame count) over all those streams' lag work, then each stream's
-// azimuthal average and the copy of its ISF to host memory. Steps do not wait for the GPU:
+// launch (per kernel instance) over all those streams' lag work (in rounds of a piece of each
+// chunk, where chunks are longer), then each stream's azimuthal average and the copy of its ISF to host memory. Steps do not wait for the GPU:
 // a stream's result is ready when a host callback queued behind its copy has run, so
 // chunks that arrive while earlier ones are on the GPU are taken by the next step.
 // (The reference analyses one video per process: src/DDM.cu:268-892.)
@@ -504,45 +504,62 @@ extern "C" int ddm_server_step(ddm_server *s, int *chunks_issued) {
     bool any = false;
     for (auto &kv : s->streams) any = any || !kv.second.pending.empty();
     if (any && (ev0 = take_event(s))) CUDA_TRY(cudaEventRecord(ev0, s->stream));
-    std::vector<std::pair<Stream *, Slot *>> taken;
-    // by round and kernel instance: a stream's launches update the same accumulators one after another
-    std::map<std::pair<int, int>, std::vector<std::pair<Stream *, DeferredLag>>> rounds;
-    // 1. each stream's next chunk: H2D copy and FFT (the engine's own stream pair), lag work deferred
+    // A chunk goes through its engine piece by piece, the lag launches of one piece queued before the FFT
+    // of the next: an engine's ring holds the longest lag and two pieces, and its FFTs wait for the lag
+    // work queued up to the piece before.
+    struct Taken {
+        Stream *st;
+        Slot *slot;
+        PendingChunk chunk;
+        int done;
+    };
+    std::vector<Taken> taken;
     for (auto &kv : s->streams) {
         Stream &st = kv.second;
         if (st.pending.empty()) continue;
-        Slot *slot = nullptr;
         for (auto &sl : st.slots)
-            if (sl->state.load() == 0) {
-                slot = sl.get();
+            if (sl->state.load() == 0) {  // else the caller has not collected earlier results yet
+                taken.push_back(Taken{&st, sl.get(), st.pending.front(), 0});
                 break;
             }
-        if (!slot) continue;  // the caller has not collected earlier results yet
-        PendingChunk pc = st.pending.front();
-        st.pending.pop_front();
-        int r = ddm_submit_frames(st.eng, pc.frames.p, pc.count, 0);
-        if (r) return r;
-        slot->frames = pc.frames;
-        slot->chunk_index = st.chunks_issued++;
-        st.frames_issued += pc.count;
-        slot->frames_done = st.frames_issued;
-        slot->submit_s = pc.submit_s;
-        slot->state.store(1);
-        st.order.push_back(slot);
-        taken.emplace_back(&st, slot);
-        int round = 0;
-        for (const DeferredLag &d : engine_take_deferred(st.eng))
-            rounds[{round++, d.EB ? hist_key(d.J, d.EB, d.CW) : d.J}].emplace_back(&st, d);
     }
-    // 2. one lag launch per kernel instance over every taken stream
-    for (auto &kv : rounds) {
-        int r = launch_batch(s, kv.second);
-        if (r) return r;
+    for (bool more = true; more;) {
+        more = false;
+        std::map<int, std::vector<std::pair<Stream *, DeferredLag>>> work;  // by kernel instance
+        // 1. each chunk's next piece: H2D copy and FFT (the engine's own stream pair), lag work deferred
+        for (Taken &t : taken) {
+            Stream &st = *t.st;
+            const int n = std::min(t.chunk.count - t.done, engine_piece_frames(st.eng));
+            if (n <= 0) continue;
+            if (t.done == 0) st.pending.pop_front();
+            int r = ddm_submit_frames(st.eng, static_cast<char *>(t.chunk.frames.p) + st.frame_bytes * t.done, n, 0);
+            if (r) return r;
+            if (t.done == 0) {
+                Slot *slot = t.slot;
+                slot->frames = t.chunk.frames;
+                slot->chunk_index = st.chunks_issued++;
+                st.frames_issued += t.chunk.count;
+                slot->frames_done = st.frames_issued;
+                slot->submit_s = t.chunk.submit_s;
+                slot->state.store(1);
+                st.order.push_back(slot);
+            }
+            t.done += n;
+            more = more || t.done < t.chunk.count;
+            // one launch at most: a piece has no more frames than a lag batch
+            for (const DeferredLag &d : engine_take_deferred(st.eng))
+                work[d.EB ? hist_key(d.J, d.EB, d.CW) : d.J].emplace_back(&st, d);
+        }
+        // 2. one lag launch per kernel instance over every stream of this round
+        for (auto &kv : work) {
+            int r = launch_batch(s, kv.second);
+            if (r) return r;
+        }
     }
     // 3. per stream: azimuthal average, ISF and status to host, completion callback
-    for (auto &ts : taken) {
-        Stream &st = *ts.first;
-        Slot *slot = ts.second;
+    for (Taken &t : taken) {
+        Stream &st = *t.st;
+        Slot *slot = t.slot;
         int r = engine_finalize_async(st.eng);
         if (r) return r;
         CUDA_TRY(cudaMemcpyAsync(slot->isf_h, engine_isf_device(st.eng), sizeof(double) * st.isf_size,

@@ -429,7 +429,8 @@ int ddm_server_add_stream(ddm_server *s, const ddm_config *cfg, int *stream_id);
 /* Remove a stream: its device memory is released once the work queued for it has run
  * (without waiting here); its unpolled results are dropped. */
 int ddm_server_remove_stream(ddm_server *s, int stream_id);
-/* Queue one chunk of `count` frames from host memory (copied; the buffer is free on return). */
+/* Queue one chunk of `count` frames (any number; a result covers the whole chunk) from host memory
+ * (copied; the buffer is free on return). */
 int ddm_server_submit(ddm_server *s, int stream_id, const void *frames, int count);
 /* As ddm_server_submit without the copy: `frames` is page-locked host memory (cudaMallocHost,
  * cudaHostRegister) that the caller leaves unchanged until this chunk's result has been
