@@ -72,13 +72,13 @@ class Server:
         """(ChunkResult fields as a dict, ISF array) of the stream's oldest finished chunk, or
         None. copy=False returns the stream's result buffer, overwritten by the next poll."""
         res, isf = self._res, self._isf[sid]
-        if copy:  # straight into the caller's array
-            isf = np.empty_like(isf)
         st = lib().ddm_server_poll(self._h, sid, C.byref(res), isf.ctypes.data, isf.size)
         if st == 0:
             return None
         if st != 1:
             raise DDMError(st, lib().ddm_last_error().decode(errors="replace"))
+        if copy:  # the array is the caller's now
+            self._isf[sid] = np.empty_like(isf)
         return {"chunk_index": res.chunk_index, "frames": res.frames, "submit_s": res.submit_s,
                 "done_s": res.done_s, "latency_s": res.done_s - res.submit_s}, isf
 
