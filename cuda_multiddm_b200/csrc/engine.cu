@@ -877,6 +877,39 @@ int run_ready_iterations(ddm_engine *e, bool final_pass) {
 
 }  // namespace
 
+namespace ddm {
+
+size_t engine_row_buffer_bytes(const ddm_engine *e) {
+    if (!e->lay.slabs || e->fft_mid) return 0;
+    const size_t frame = sizeof(float2) * e->lay.E;
+    return frame * std::min<size_t>(e->jmax, (256u << 20) / frame);
+}
+
+size_t engine_take_row_buffer(ddm_engine *e) {
+    const size_t bytes = engine_row_buffer_bytes(e);
+    if (!bytes) return 0;
+    // in the order of the one stream that uses it: no wait for passes already queued there
+    if (cudaMallocAsync(reinterpret_cast<void **>(&e->fft_mid), bytes, e->fft_stream) != cudaSuccess) {
+        e->fft_mid = nullptr;
+        cudaGetLastError();
+        return 0;
+    }
+    e->device_bytes += bytes;
+    e->fft_mid_frames = static_cast<int>(bytes / (sizeof(float2) * e->lay.E));
+    return bytes;
+}
+
+cudaStream_t engine_drop_row_buffer(ddm_engine *e) {
+    if (!e->fft_mid) return nullptr;
+    e->device_bytes -= sizeof(float2) * e->lay.E * e->fft_mid_frames;
+    cudaFreeAsync(e->fft_mid, e->fft_stream);  // only that stream's passes use it
+    e->fft_mid = nullptr;
+    e->fft_mid_frames = 0;
+    return e->fft_stream;
+}
+
+}  // namespace ddm
+
 // =================================================================================
 // C ABI
 // =================================================================================
@@ -1097,22 +1130,6 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
     }
     if ((st = dev_alloc(e, &e->acc, static_cast<size_t>(e->T) * e->lay.E))) return bail(st);
     if ((st = dev_alloc(e, &e->stage, stage_bytes))) return bail(st);
-    if (e->lay.slabs) {
-        // The row pass's output of one FFT group, in frame order: at most 256 MB. Not part of the budget
-        // check: left out where it does not fit.
-        const size_t frame = sizeof(float2) * e->lay.E;
-        const int frames = static_cast<int>(std::min<size_t>(e->jmax, (256u << 20) / frame));
-        const size_t bytes = frame * frames;
-        if (frames > 0 && (!cfg->hbm_budget_bytes || need + bytes <= cfg->hbm_budget_bytes)) {
-            if (dev_alloc(e, &e->fft_mid, static_cast<size_t>(frames) * e->lay.E) == DDM_OK) {
-                e->fft_mid_frames = frames;
-            } else {
-                e->fft_mid = nullptr;
-                cudaGetLastError();
-                clear_error();
-            }
-        }
-    }
     if ((st = dev_alloc(e, &e->tables_d, static_cast<size_t>(kTables) * e->tab_stride))) return bail(st);
     if ((st = dev_alloc(e, &e->norm_d, 2 * e->T))) return bail(st);
     if ((st = dev_alloc(e, &e->isf_d, e->isf_size))) return bail(st);
@@ -1239,6 +1256,10 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
         (compat && cudaMemsetAsync(e->ring, 0, sizeof(float2) * e->R * e->lay.E, e->fft_stream) != cudaSuccess) ||
         (e->own_stream && cudaStreamSynchronize(e->fft_stream) != cudaSuccess))
         return bail(fail(DDM_ERR_CUDA, "initial memset failed"));
+    // Not part of the budget check, and after every buffer the engine cannot do without: left out where
+    // it does not fit.
+    const size_t mid = engine_row_buffer_bytes(e);
+    if (mid && (!cfg->hbm_budget_bytes || need + mid <= cfg->hbm_budget_bytes)) engine_take_row_buffer(e);
     *out = e;
     return DDM_OK;
 }

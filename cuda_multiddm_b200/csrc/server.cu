@@ -65,7 +65,8 @@ struct PendingChunk {
 struct Stream {
     ddm_engine *eng = nullptr;
     cudaEvent_t gone = nullptr;  // removal: recorded after the stream's last queued work
-    size_t bytes = 0;
+    size_t bytes = 0;       // device memory the stream needs
+    size_t row_buffer = 0;  // and its FFT row buffer, given back when another stream needs the room
     size_t frame_bytes = 0;
     long isf_size = 0;
     long chunks_submitted = 0, chunks_issued = 0, frames_issued = 0;
@@ -93,7 +94,8 @@ void CUDART_CB on_result(void *arg) {  // runs on a CUDA driver thread: no CUDA 
 struct ddm_server {
     int device = 0, sms = 0;
     cudaStream_t stream = nullptr;
-    size_t budget = 0, used = 0, reserved = 0;
+    size_t budget = 0, used = 0, reserved = 0;  // used: without the row buffers
+    size_t row_buffers = 0;
     int opening = 0;  // streams being admitted outside the lock
     int max_streams = 64, results_per_stream = 4;
     Clock::time_point t0 = Clock::now();
@@ -140,6 +142,37 @@ void reap(ddm_server *s, bool wait) {
         } else {
             ++it;
         }
+    }
+}
+
+size_t room(const ddm_server *s) {  // of the budget, with every row buffer given back
+    const size_t taken = s->used + s->reserved;
+    return taken < s->budget ? s->budget - taken : 0;
+}
+
+// Row buffers are given back until the budget holds what is used and reserved; the returned streams
+// free their memory.
+std::vector<cudaStream_t> make_room(ddm_server *s) {
+    std::vector<cudaStream_t> freeing;
+    for (auto &kv : s->streams) {
+        if (s->row_buffers <= room(s)) break;
+        Stream &st = kv.second;
+        if (!st.row_buffer) continue;
+        freeing.push_back(engine_drop_row_buffer(st.eng));
+        s->row_buffers -= st.row_buffer;
+        st.row_buffer = 0;
+    }
+    return freeing;
+}
+
+// Streams without a row buffer get one while the budget has room for it.
+void give_row_buffers(ddm_server *s) {
+    for (auto &kv : s->streams) {
+        Stream &st = kv.second;
+        const size_t bytes = engine_row_buffer_bytes(st.eng);
+        if (!bytes || s->row_buffers + bytes > room(s)) continue;
+        st.row_buffer = engine_take_row_buffer(st.eng);
+        s->row_buffers += st.row_buffer;
     }
 }
 
@@ -368,6 +401,8 @@ extern "C" int ddm_server_add_stream(ddm_server *s, const ddm_config *cfg, int *
     size_t need = 0;
     int r = engine_plan_bytes(&c, &need);
     if (r) return r;
+    c.hbm_budget_bytes = need;  // no row buffer yet
+    std::vector<cudaStream_t> freeing;
     // admission: reserve the stream's bytes under the lock, build its engine without it (steps
     // of the admitted streams go on meanwhile), then insert it
     {
@@ -375,14 +410,14 @@ extern "C" int ddm_server_add_stream(ddm_server *s, const ddm_config *cfg, int *
         reap(s, false);
         if (static_cast<int>(s->streams.size()) + s->opening >= s->max_streams)
             return fail(DDM_ERR_BUSY, "all stream slots are taken");
-        if (s->used + s->reserved + need > s->budget)
+        if (need > room(s))
             return fail(DDM_ERR_BUSY, "not admitted now: the stream needs " + std::to_string(need) +
-                                          " device bytes, " + std::to_string(s->budget - s->used - s->reserved) +
-                                          " of the budget are free");
-        c.hbm_budget_bytes = s->budget - s->used - s->reserved;  // for the engine's optional buffers
+                                          " device bytes, " + std::to_string(room(s)) + " of the budget are free");
         s->reserved += need;
         s->opening++;
+        freeing = make_room(s);
     }
+    for (cudaStream_t f : freeing) cudaStreamSynchronize(f);
     Stream st;
     auto unreserve = [&]() {
         std::lock_guard<std::mutex> g(s->lock);
@@ -427,6 +462,8 @@ extern "C" int ddm_server_add_stream(ddm_server *s, const ddm_config *cfg, int *
     s->used += st.bytes;
     const int id = s->next_id++;
     s->streams.emplace(id, std::move(st));
+    make_room(s);  // the engine's bytes may come to a little more than its plan
+    give_row_buffers(s);
     *stream_id = id;
     return DDM_OK;
 }
@@ -447,8 +484,12 @@ extern "C" int ddm_server_remove_stream(ddm_server *s, int stream_id) {
         st.gone = nullptr;
         CUDA_TRY(cudaStreamSynchronize(s->stream));
     }
+    engine_drop_row_buffer(st.eng);
+    s->row_buffers -= st.row_buffer;
+    st.row_buffer = 0;
     s->closing.push_back(std::move(st));
     reap(s, false);
+    give_row_buffers(s);
     return DDM_OK;
 }
 
@@ -624,7 +665,7 @@ extern "C" int ddm_server_get_stats(const ddm_server *s, ddm_server_stats *info)
     if (!s || !info) return fail(DDM_ERR_INVALID_ARG, "bad argument");
     std::lock_guard<std::mutex> g(s->lock);
     info->streams = static_cast<int>(s->streams.size());
-    info->device_bytes = s->used;
+    info->device_bytes = s->used + s->row_buffers;
     info->budget_bytes = s->budget;
     info->batched_launches = s->launches;
     long pending = 0;
