@@ -882,7 +882,7 @@ namespace ddm {
 size_t engine_row_buffer_bytes(const ddm_engine *e) {
     if (!e->lay.slabs || e->fft_mid) return 0;
     const size_t frame = sizeof(float2) * e->lay.E;
-    return frame * std::min<size_t>(e->jmax, (256u << 20) / frame);
+    return frame * std::min<size_t>(e->jmax, std::max<size_t>(e->fft_group, (256u << 20) / frame));
 }
 
 size_t engine_take_row_buffer(ddm_engine *e) {

@@ -36,9 +36,10 @@ struct LagTarget {  // what a lag launch of this engine reads and writes
 // for the caller to issue, on the engine's stream, after the work queued before them.
 void engine_defer_lag(ddm_engine *e, bool on);
 std::vector<DeferredLag> engine_take_deferred(ddm_engine *e);
-// The buffer for the FFT row pass's output ([frame][element], at most 256 MB; without it the pass works in
-// the ring): what it would take (0: not used, or there already); allocates it (bytes, or 0); frees it
-// in the order of the returned stream, on which a caller waits for the memory to be free.
+// The buffer for the FFT row pass's output ([frame][element]: what 256 MB hold, or fft_group_frames if that
+// is more; without it the pass works in the ring): what it would take (0: not used, or there already);
+// allocates it (bytes, or 0); frees it in the order of the returned stream, on which a caller waits for
+// the memory to be free.
 size_t engine_row_buffer_bytes(const ddm_engine *e);
 size_t engine_take_row_buffer(ddm_engine *e);
 cudaStream_t engine_drop_row_buffer(ddm_engine *e);

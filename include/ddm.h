@@ -96,8 +96,7 @@ typedef struct {
                                       (both within 1e-5 of the FP64 oracle). With
                                       lag_batch_frames = -1 the tuned geometry is used. */
     int fft_group_frames;          /* frames per FFT launch (both passes over every scale);
-                                      0, and the most a launch takes = as many as 256 MB of
-                                      spectra hold (at least 1). With
+                                      0 = as many as 256 MB of spectra hold (at least 1). With
                                       lag_batch_frames = -1 the tuned value is used. */
     int fft_per_tile;              /* 1: tiles of side 32..128 are transformed by one kernel that
                                       keeps each tile in shared memory between its row and column
