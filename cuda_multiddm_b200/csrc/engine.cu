@@ -1427,7 +1427,9 @@ std::vector<DeferredLag> engine_take_deferred(ddm_engine *e) {
 
 int engine_piece_frames(const ddm_engine *e) { return e->jmax; }
 
-LagTarget engine_lag_target(const ddm_engine *e) { return LagTarget{e->ring, e->acc, e->E, e->status_d, &e->maps}; }
+LagTarget engine_lag_target(const ddm_engine *e) {
+    return LagTarget{e->ring, e->acc, e->E, e->status_d, e->hist.EB ? nullptr : &e->maps};
+}
 
 HistTarget engine_hist_target(const ddm_engine *e) {
     return HistTarget{e->ring, e->acc, e->lay, e->T, e->status_d, e->wait_cycles};

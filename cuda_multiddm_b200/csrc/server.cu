@@ -70,7 +70,7 @@ struct Stream {
     size_t frame_bytes = 0;
     long isf_size = 0;
     long chunks_submitted = 0, chunks_issued = 0, frames_issued = 0;
-    LagMaps *maps_d = nullptr;
+    LagMaps *maps_d = nullptr;  // of the ring lag kernel (engines on the other one have none)
     LagMaps *maps_h = nullptr;  // pinned source of the maps_d upload
     std::deque<PendingChunk> pending;
     std::vector<std::unique_ptr<Slot>> slots;
@@ -211,7 +211,7 @@ int pinned(PinnedBuf *b, size_t bytes) {
 // Releases a stream whose queued work has all run (its removal event has completed).
 void release_stream(Stream &st) {
     engine_close_async(st.eng);
-    cudaFreeAsync(st.maps_d, nullptr);
+    if (st.maps_d) cudaFreeAsync(st.maps_d, nullptr);
     pinned_release(st.maps_h);
     for (auto &sl : st.slots) {
         pinned_release(sl->isf_h);
@@ -435,14 +435,16 @@ extern "C" int ddm_server_add_stream(ddm_server *s, const ddm_config *cfg, int *
     st.bytes = info.device_bytes;
     st.frame_bytes = static_cast<size_t>(cfg->frame_width) * cfg->frame_height * cfg->bytes_per_pixel;
     st.isf_size = ddm_isf_size(st.eng);
-    const LagTarget t = engine_lag_target(st.eng);
-    // the tensor maps go up from page-locked memory: a copy from pageable memory may wait for
-    // the shared stream to drain, holding up this call and the steps' launches meanwhile
-    st.maps_h = static_cast<LagMaps *>(pinned_alloc(sizeof(LagMaps)));
-    bool ok = st.maps_h != nullptr;
-    if (ok) *st.maps_h = *t.maps;
-    ok = ok && cudaMallocAsync(reinterpret_cast<void **>(&st.maps_d), sizeof(LagMaps), s->stream) == cudaSuccess &&
-         cudaMemcpyAsync(st.maps_d, st.maps_h, sizeof(LagMaps), cudaMemcpyHostToDevice, s->stream) == cudaSuccess;
+    bool ok = true;
+    if (const LagMaps *maps = engine_lag_target(st.eng).maps) {
+        // the tensor maps go up from page-locked memory: a copy from pageable memory may wait for
+        // the shared stream to drain, holding up this call and the steps' launches meanwhile
+        st.maps_h = static_cast<LagMaps *>(pinned_alloc(sizeof(LagMaps)));
+        ok = st.maps_h != nullptr;
+        if (ok) *st.maps_h = *maps;
+        ok = ok && cudaMallocAsync(reinterpret_cast<void **>(&st.maps_d), sizeof(LagMaps), s->stream) == cudaSuccess &&
+             cudaMemcpyAsync(st.maps_d, st.maps_h, sizeof(LagMaps), cudaMemcpyHostToDevice, s->stream) == cudaSuccess;
+    }
     for (int i = 0; ok && i < s->results_per_stream; i++) {
         auto sl = std::make_unique<Slot>();
         sl->server = s;
