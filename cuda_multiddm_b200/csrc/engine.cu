@@ -390,12 +390,14 @@ int launch_fft(ddm_engine *e, const uint8_t *src, long long frame_stride, long l
         smem = std::max(smem, fft_smem_bytes(s));
     }
     rows.S = cols.S = nfft;
-    // The column pass writes neighbouring lines of a slab for neighbouring frames, so its CTAs take the
-    // frames of a few columns together (30 frames of 1024^2, four scales: 0.498 -> 0.462 ms).
-    // Groups that stay in L2 gain nothing from it.
-    constexpr double kFramesFirstMin = 32.0 * (1 << 20);
+    // The column pass writes neighbouring lines of a slab for neighbouring frames. Its CTAs take the frames
+    // of a few columns together where frames are so large that a group holds few of them (both passes,
+    // alone, 30 frames: 2048^2 with seven scales 3816 us against 3770, four 2388 / 2369). With smaller
+    // frames the columns of one frame after another are faster (2048^2, one scale 760 / 838; 1024^2, four
+    // scales 499 / 504, two 275 / 291, one 157 / 173; 512^2, four 124 / 127, one 49.6 / 51.1).
+    constexpr double kFramesFirstMin = 64e6;  // bytes of a frame's spectra
     cols.frames_first = e->lay.slabs && e->fft_mid && col_ctas <= 65535 &&
-                        static_cast<double>(sizeof(float2)) * e->E * nframes >= kFramesFirstMin;
+                        static_cast<double>(sizeof(float2)) * e->E >= kFramesFirstMin;
     // Frames go through both passes in groups of up to 256 MB of spectra (15 frames of the
     // 1024^2 x 4-scale shape): fewer, larger launches were measured faster than groups small
     // enough for the row pass's output to stay in L2 (frames/s at 34 / 64 / 100 / 256 MB:
