@@ -588,14 +588,15 @@ int launch_hist(ddm_engine *e, const Launch &L) {
         return DDM_OK;
     }
     const HistTarget target{e->ring, e->acc, e->lay, e->T, e->status_d, e->wait_cycles};
+    const size_t smem = hist_launch_smem(table.smem, e->M, e->E);
     TimedRange tr(e, 1);
     switch (hist_key(J, EB, CW)) {
 #define HIST_CASE(JJ, BB, WW)                                                                                     \
     case hist_key(JJ, BB, WW): {                                                                                  \
-        const int per_sm = lag_resident_ctas(e, (1 << 20) + hist_key(JJ, BB, WW), table.smem,                    \
+        const int per_sm = lag_resident_ctas(e, (1 << 20) + hist_key(JJ, BB, WW), smem,                          \
                                              lag_hist_kernel<JJ, BB, WW>, hist_threads(WW));                     \
         const unsigned grid = balanced_grid(blocks, static_cast<unsigned>(per_sm * e->sms));                     \
-        lag_hist_kernel<JJ, BB, WW><<<grid, hist_threads(WW), table.smem, e->stream>>>(                           \
+        lag_hist_kernel<JJ, BB, WW><<<grid, hist_threads(WW), smem, e->stream>>>(                                 \
             target, td, static_cast<int>(blocks), inl);                                                           \
         break;                                                                                                    \
     }

@@ -327,6 +327,19 @@ inline bool hist_always_fits(const HistInput &steady, const HistShape &shape, bo
     return false;
 }
 
+// Dynamic shared memory a launch asks for, given what its table needs. Three CTAs of up to 54 KB take the
+// same split of an SM's memory as the FFT passes' CTAs (164 KB), and the next piece's FFT, queued at the
+// same time, then mixes with a lag launch that needs all of its CTAs at once. For frames of up to 512^2 the two
+// took longer than one after the other (192 frames in submits of 32, 512^2, four scales: 24 taus up to 600
+// 3213 us, with 56,000 bytes 2504, ring kernel 2558; 64 up to 300 3030 / 2855; 20 up to 1000 2622 / 2488;
+// two scales: 1709 / 1542, 1410 / 1348, 1404 / 1334). Larger frames measured the same either way (1024^2, one
+// to four scales: within 1 %), small launches gain from the mixing (256^2, three scales: 3 - 4 %; 512^2, one: 1 %).
+inline size_t hist_launch_smem(size_t table_smem, int side, long long E) {
+    constexpr size_t kOwnSplit = 56000;
+    constexpr long long kMinElements = 200000;
+    return side <= 512 && E >= kMinElements ? std::max(table_smem, kOwnSplit) : table_smem;
+}
+
 // The shape for launches like `steady` (every partner there): as many CTAs per SM as the rows
 // leave room for, with the widest block (a thread of a wider block walks more entries per load of
 // its register frames), and in their shared memory whole blocks in two or more row buffers, else

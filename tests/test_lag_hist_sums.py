@@ -45,6 +45,8 @@ def batches(calls, chunk):
     (512, [512, 256, 128, 64], media.log_taus(1, 90, 40), 30, (150, 64, 31)),
     (512, [512, 256, 128, 64], RUNS, 32, (150, 64, 95)),
     (256, [256, 128], media.log_taus(1, 620, 64), 17, (600, 130)),
+    (512, [512, 256], media.log_taus(1, 300, 64), 32, (310, 64, 32, 9)),  # launches that ask for more shared memory
+    (512, [512, 256], list(range(1, 21)), 30, (75, 40)),                  # than their tables need
 ])
 def test_sums_match_float64_and_the_ring_kernel(side, scales, taus, chunk, calls):
     rng = np.random.default_rng(side + chunk)
