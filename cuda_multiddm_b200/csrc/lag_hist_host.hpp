@@ -347,13 +347,17 @@ inline size_t hist_launch_smem(size_t table_smem, int side, long long E) {
 // rows are there) comes after the narrower block: 32-frame launches of 512^2, four scales, 64 taus
 // up to 300, took 569 us with it, 514 in the ring kernel and 430 with blocks of 16 and
 // register-frame buffers. The ring kernel keeps short tau lists, whose blocks are too little work for
-// their barriers (5 taus up to 20: 130 us against 142), and those that one CTA per SM would run
-// without many taus (20 taus up to 1000: 393 us against 439; 64: 727 against 648).
+// their barriers (5 taus up to 20: 130 us against 142), and those that one CTA per SM would run without
+// many taus: its one row buffer is loaded for little work (192 frames of 512^2, two scales, submits of 32,
+// ring kernel / this: 100 taus up to 1300 3247 us / 3640, 80 up to 1650 2930 / 3600; 128 up to 1000 3550 / 3407,
+// up to 1300 4320 / 3614). Launches of two batches save more reads (against single batches: 48 up to 1300
+// 1997 / 2416, 64 up to 1000 2110 / 2427, 80 2256 / 2517; 100 up to 1000 2817 / 2648, 128 3407 / 2676).
 // A shape is taken only if no launch of the engine can outgrow it (hist_always_fits): the ring's
 // layout follows the kernel, so there is no other one to go to later.
 inline HistShape hist_pick_shape(const HistInput &steady, bool scattered) {
-    constexpr int kMinTaus = 8, kMinTausOneCta = 48;
-    constexpr struct {
+    constexpr int kMinTaus = 8;
+    const int kMinTausOneCta = steady.nsub > 1 ? 96 : 112;
+    const struct {
         int EB, CW, taus;
         bool bare;
     } sizes[] = {{32, 4, kMinTaus, false}, {16, 4, kMinTaus, true}, {16, 6, kMinTaus, true}, {16, 12, kMinTausOneCta, true}};
