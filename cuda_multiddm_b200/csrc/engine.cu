@@ -231,6 +231,11 @@ int dev_alloc(ddm_engine *e, Tp **p, size_t count) {
     // stream-ordered from the device's memory pool (no device-wide synchronisation when
     // engines come and go), on the engine's private FFT stream, complete before it is used
     cudaError_t err = cudaMallocAsync(reinterpret_cast<void **>(p), bytes, e->fft_stream);
+    if (err == cudaErrorMemoryAllocation && engine_drop_row_buffer(e)) {  // the optional buffer makes room
+        cudaGetLastError();
+        err = cudaStreamSynchronize(e->fft_stream);
+        if (err == cudaSuccess) err = cudaMallocAsync(reinterpret_cast<void **>(p), bytes, e->fft_stream);
+    }
     if (err == cudaSuccess) err = cudaStreamSynchronize(e->fft_stream);
     if (err != cudaSuccess)
         return fail(DDM_ERR_OUT_OF_MEMORY, std::string("cudaMalloc of ") + std::to_string(bytes) +
@@ -1133,6 +1138,10 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
     }
     if ((st = dev_alloc(e, &e->acc, static_cast<size_t>(e->T) * e->lay.E))) return bail(st);
     if ((st = dev_alloc(e, &e->stage, stage_bytes))) return bail(st);
+    // Not part of the budget check: left out where it does not fit, and given up if another buffer does not
+    // fit beside it (dev_alloc).
+    const size_t mid = engine_row_buffer_bytes(e);
+    if (mid && (!cfg->hbm_budget_bytes || need + mid <= cfg->hbm_budget_bytes)) engine_take_row_buffer(e);
     if ((st = dev_alloc(e, &e->tables_d, static_cast<size_t>(kTables) * e->tab_stride))) return bail(st);
     if ((st = dev_alloc(e, &e->norm_d, 2 * e->T))) return bail(st);
     if ((st = dev_alloc(e, &e->isf_d, e->isf_size))) return bail(st);
@@ -1259,10 +1268,6 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
         (compat && cudaMemsetAsync(e->ring, 0, sizeof(float2) * e->R * e->lay.E, e->fft_stream) != cudaSuccess) ||
         (e->own_stream && cudaStreamSynchronize(e->fft_stream) != cudaSuccess))
         return bail(fail(DDM_ERR_CUDA, "initial memset failed"));
-    // Not part of the budget check, and after every buffer the engine cannot do without: left out where
-    // it does not fit.
-    const size_t mid = engine_row_buffer_bytes(e);
-    if (mid && (!cfg->hbm_budget_bytes || need + mid <= cfg->hbm_budget_bytes)) engine_take_row_buffer(e);
     *out = e;
     return DDM_OK;
 }
