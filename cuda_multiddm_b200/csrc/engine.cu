@@ -1103,7 +1103,8 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
         return bail(fail(DDM_ERR_CUDA, "stream/event creation failed"));
     // Launches of up to 32 frames of geometry 0 run on the resident-history kernel where their
     // frames fit its shared memory, on a ring in slabs; the ring kernel keeps the others.
-    if (e->lag_geom == 0 && e->lag_batch <= kHistMaxJ) {
+    if (e->lag_geom == 0 && e->lag_batch <= kHistMaxJ &&
+        (compat || !hist_leave_to_ring(e->E, e->S, e->tau_max, e->C))) {
         e->hist = hist_pick_shape(hist_steady(e->taus, e->lag_batch, 1, e->R, compat), compat);
         if (e->hist.EB)
             e->tab_stride = std::max(e->tab_stride, hist_table_capacity(e->T, e->tau_max + e->lag_batch, 1));

@@ -327,6 +327,20 @@ inline bool hist_always_fits(const HistInput &steady, const HistShape &shape, bo
     return false;
 }
 
+// Whether lags below 40 of very large frames in one or two scales are left to the ring kernel: its launches
+// take no more time there, and the FFT writes whole frames faster than slabs (192 frames of 2048^2, two
+// scales, ring kernel / this: 16 taus up to 28 12.0 ms / 13.3, 20 up to 20 12.0 / 13.1, 12 up to 32 11.8 / 12.7,
+// 24 up to 32 13.4 / 14.1; 24 up to 40 14.9 / 14.1). With more scales the FFT's share is smaller (four, 12 up to 20
+// 21.7 / 21.3; six, 14 up to 22 33.1 / 31.8), and smaller frames go either way by a few percent (1024^2, four
+// scales, 20 up to 20 5.6 / 5.8, up to 30 5.6 / 5.4; 512^2, four, 12 up to 20 1374 us / 1257). Not where a chunk
+// ends in a launch of a frame count without an instance, which the ring kernel runs masked (chunks of 25:
+// 12.4 ms / 10.6).
+inline bool hist_leave_to_ring(long long E, int scales, int tau_max, int chunk) {
+    constexpr long long kMinElements = 1LL << 22;
+    const int rest = chunk < kHistMaxJ ? chunk : chunk % kHistMaxJ;
+    return E >= kMinElements && scales <= 2 && tau_max < 40 && (rest == 0 || hist_pick_j(rest) == rest);
+}
+
 // Dynamic shared memory a launch asks for, given what its table needs. Three CTAs of up to 54 KB take the
 // same split of an SM's memory as the FFT passes' CTAs (164 KB), and the next piece's FFT, queued at the
 // same time, then mixes with a lag launch that needs all of its CTAs at once. For frames of up to 512^2 the two
