@@ -401,6 +401,7 @@ extern "C" int ddm_server_add_stream(ddm_server *s, const ddm_config *cfg, int *
     size_t need = 0;
     int r = engine_plan_bytes(&c, &need);
     if (r) return r;
+    if (cudaSetDevice(s->device) != cudaSuccess) return fail(DDM_ERR_NO_DEVICE, "cudaSetDevice failed");
     c.hbm_budget_bytes = need;  // no row buffer yet
     std::vector<cudaStream_t> freeing;
     // admission: reserve the stream's bytes under the lock, build its engine without it (steps
