@@ -1110,9 +1110,11 @@ int open_engine(const ddm_config *cfg, ddm_engine **out, size_t *need_out, bool 
             e->tab_stride = std::max(e->tab_stride, hist_table_capacity(e->T, e->tau_max + e->lag_batch, 1));
         // Two batches per launch where the ring holds both and the batches do not depend on how the
         // frames arrive (a batch smaller than the ingest piece is cut at every piece). 64 taus up to 500
-        // at 1024^2, four scales: 1.85 ms per 32 frames one by one, 1.40 in pairs. Small launches gain
-        // more from running beside the next piece's FFT, which must wait for the longer launch (200
-        // frames of 256^2, 20 taus: 233 us one by one, 253 in pairs).
+        // at 1024^2, four scales: 1.66 ms per 32 frames one by one, 1.40 in pairs. Small launches gain
+        // more from running beside the next piece's FFT, which must wait for the longer launch. Gain of
+        // pairs over 96 / 200 / 480 frames in one call, by elements x taus: 0.66e6 0.97 / 0.87 / 0.87,
+        // 2.7e6 1.01 / 1.02 / 1.04, 4.8e6 0.99 / 1.01 / 0.99, 6.3e6 1.01 / 0.98 / 0.97, 8.4e6 1.03 / 1.02 / 1.02,
+        // 12.6e6 1.01 / 1.00 / 1.00, 17e6 1.04 / 1.06 / 1.05, 34e6 1.20 / 1.15 / 1.11, 67e6 1.06 / 1.08 / 1.16.
         constexpr double kPairMinWork = 16e6;  // elements x taus: about 150 us per launch
         if (e->hist.EB && !compat && e->G == 0 && e->lag_batch >= e->jmax &&
             e->R - e->tau_max >= 2 * e->lag_batch && static_cast<double>(e->E) * e->T >= kPairMinWork) {

@@ -38,6 +38,8 @@ struct ScaleDesc {
 // has fewer warps than the GPU holds (a chunk is a serial chain of gathers: 256^2, 20 taus, 10
 // lambdas took 16 us with chunks of 1024).
 constexpr int kAzChunk = 1024, kAzMinChunk = 128;
+// A B200's 148 SMs times 32 warps; fixed, not the device's own count, because the chunk sets the order of the
+// FP64 sums: one configuration has the same bits everywhere.
 constexpr long long kAzWantWarps = 148 * 32;
 constexpr int kAzWarps = kAzThreads / 32;
 

@@ -31,11 +31,12 @@
 // prefetched into L2 by the producer and read at the start of an entry, used at its end.
 //
 // What bounds it, measured (32 frames, 1024^2 with four scales, launch alone; ring kernel beside it):
-// 64 taus up to 500 1.69 ms = 6.2 TB/s, 0.95 of the copy bandwidth (2.03 ms), with two batches per
+// 64 taus up to 500 1.66 ms = 6.3 TB/s, 0.96 of the copy bandwidth (2.03 ms), with two batches per
 // launch 1.40 ms per 32 frames, bound by issue and latency of the pairs (issue slots 48 %, shared-memory
-// pipe 45 %); 64 taus up to 200 1.37 ms (1.56), 48 up to 100 0.86 ms (1.14), 20 up to 30 0.40 ms (0.45),
-// bound by the pairs. Slower and not used: runs of eight taus and a loop per kind of unit (1.85 -> 2.30 ms
-// beside the FFT, instruction fetch), the next unit's table entry loaded ahead (+1 to +5 %).
+// pipe 45 %); 64 taus up to 200 1.40 ms (1.56), 48 up to 100 0.89 ms (1.14), 20 up to 30 0.41 ms (0.45),
+// bound by the pairs. Slower and not used, in an earlier form of the kernel: runs of eight taus and a loop
+// per kind of unit (1.85 -> 2.30 ms beside the FFT, instruction fetch), the next unit's table entry loaded
+// ahead (+1 to +5 %).
 //
 // Sub-batches whose lists differ (the first frames of a stream, where partners are missing) are
 // separated by a barrier of the consumer warps, since another thread may then own an entry's
@@ -48,7 +49,7 @@
 
 namespace ddm {
 
-constexpr int kHistMaxSub = 4;                   // sub-batches per launch at most
+constexpr int kHistMaxSub = 4;  // sub-batches per launch that tables and barriers have room for (engines use one or two)
 constexpr int kHistJs[] = {4, 8, 16, 20, 24, 30, 32};
 constexpr int kHistMaxJ = 32;
 constexpr int kHistRowBytes = 128;  // 16 elements

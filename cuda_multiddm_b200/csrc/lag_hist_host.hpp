@@ -361,8 +361,10 @@ inline size_t hist_launch_smem(size_t table_smem, int side, long long E) {
 // rows are there) comes after the narrower block: 32-frame launches of 512^2, four scales, 64 taus
 // up to 300, took 569 us with it, 514 in the ring kernel and 430 with blocks of 16 and
 // register-frame buffers. The ring kernel keeps short tau lists, whose blocks are too little work for
-// their barriers (5 taus up to 20: 130 us against 142), and those that one CTA per SM would run without
-// many taus: its one row buffer is loaded for little work (192 frames of 512^2, two scales, submits of 32,
+// their barriers (192 frames in submits of 32, with the FFT, per 32, ring kernel / this: 1024^2, four scales, 6 taus
+// up to 20 756 us / 800, up to 100 867 / 849, 8 up to 20 791 / 809, up to 100 925 / 885, up to 300 1006 / 1068, 10 up
+// to 100 961 / 919; 512^2, four scales, 6 up to 20 154 / 162, 8 up to 20 161 / 164, up to 100 190 / 186), and those
+// that one CTA per SM would run without many taus: its one row buffer is loaded for little work (192 frames of 512^2, two scales, submits of 32,
 // ring kernel / this: 100 taus up to 1300 3247 us / 3640, 80 up to 1650 2930 / 3600; 128 up to 1000 3550 / 3407,
 // up to 1300 4320 / 3614). Launches of two batches save more reads (against single batches: 48 up to 1300
 // 1997 / 2416, 64 up to 1000 2110 / 2427, 80 2256 / 2517; 100 up to 1000 2817 / 2648, 128 3407 / 2676).
